@@ -52,11 +52,13 @@ typedef struct fdtd_stats {
   int64_t e_split_cells; /* cells whose E components are stored as split fields */
   int64_t h_split_cells; /* cells whose H components are stored as split fields */
   int n_tiles;           /* thread blocks per time step */
-  int64_t step_launches; /* time-step kernel launches issued by the last run */
+  int64_t step_launches; /* time-step kernel launches issued by the last run (a launch of the resident
+                            kernel advances many steps and counts once per step) */
   int64_t dft_launches;  /* DFT kernel launches issued by the last run */
   double last_run_ms;    /* device time of the last run (CUDA events) */
   double compile_ms;     /* host time spent building the material table */
-  int variant;           /* step kernel: 0 plain loads, 1 TMA streaming */
+  int variant;           /* step kernel: 0 plain loads, 1 TMA streaming, 2 resident (tile_y, stages, zchunk:
+                            its bricks along x, y, z) */
   int tile_y;            /* tile height (rows) of the step kernel */
   int stages;            /* shared-memory pipeline stages (TMA kernel) */
   int zchunk;            /* z planes per tile */
@@ -140,7 +142,10 @@ int fdtd_synchronize(fdtd_sim* s);
  * per tile (0: derived from the grid). tile_y = 0 with variant 1 autotunes:
  * the first run times a few candidate (tile_y, stages, zchunk, one or two
  * tile lists) shapes on the simulation itself for a few steps and keeps the
- * fastest, remembered per set of grid sizes for the life of the process. The
+ * fastest, remembered per set of grid sizes for the life of the process. A
+ * single grid whose state fits in the GPU's shared memory, without monitors
+ * and without anything kept for a gradient, is then stepped by the resident
+ * kernel (one cooperative launch for many steps; its partitions are timed). The
  * default comes from RFN_FDTD_KERNEL (plain / stream) / RFN_FDTD_TY /
  * RFN_FDTD_STAGES / RFN_FDTD_ZCHUNK or is (1, 0, 6, 0): autotuned streaming.
  * RFN_FDTD_ONE_LIST=1 sends the plain tiles of an explicit streaming shape

@@ -29,6 +29,7 @@
 #include "fdtd_adjoint.cuh"
 #include "fdtd_nf2ff.cuh"
 #include "fdtd_step_stream.cuh"
+#include "fdtd_resident.cuh"
 #include "fdtd_adjoint_stream.cuh"
 #include <cudaTypedefs.h>
 
@@ -37,6 +38,7 @@ using namespace rfn;
 namespace {
 
 constexpr int kDftChunk = 256;  // steps between DFT accumulation passes
+constexpr int kResidentSteps = 16 * kDftChunk;  // most steps of one launch of the resident kernel
 constexpr int kMaxProbes = 1 << 20;
 constexpr int kMaxMonitors = 50;  // MAX_MONITORS, rfnetwork/core/inc/solver.h:15
 
@@ -136,10 +138,10 @@ int threads_for_host() {
 // Kernel selection of an engine: the plain-load kernel (one cell per thread)
 // or the TMA-pipelined streaming kernel (tile height, plane slots), and the z chunk.
 struct KernelConfig {
-  int variant = 1;  // 0 plain loads, 1 TMA streaming
-  int ty = 0;       // tile height; 0 (with variant 1): autotuned (ty, stages, zchunk)
-  int stages = 6;   // streaming: shared-memory plane slots
-  int zchunk = 0;   // 0: pick from the grid size
+  int variant = 1;  // 0 plain loads, 1 TMA streaming, 2 resident (only ever the engine's own choice)
+  int ty = 0;       // tile height; 0 (with variant 1): autotuned (ty, stages, zchunk); resident: bricks along x
+  int stages = 6;   // streaming: shared-memory plane slots; resident: bricks along y
+  int zchunk = 0;   // 0: pick from the grid size; resident: bricks along z
   int one_list = 0; // streaming: every tile through the general instantiation (no plain-tile kernel beside it)
 };
 
@@ -439,10 +441,33 @@ struct StreamClass {
   }
 };
 
+// Everything one launch of the resident kernel needs.
+struct ResidentClass {
+  ResGrid g{};
+  int threads = 0, faces = 0, blocks = 0;
+  uint32_t smem = 0;
+  DevBuf<uint2> lists;               // E lists, H lists, E face words, H face words
+  DevBuf<int4> count;
+  DevBuf<uint16_t> stride, row_ids;
+  DevBuf<unsigned long long> face;   // E faces, then H faces
+  void reset() {
+    blocks = 0;
+    lists.free();
+    count.free();
+    stride.free();
+    row_ids.free();
+    face.free();
+  }
+};
+
+constexpr uint32_t kResSmemMax = 232448 - 1024;  // dynamic shared bytes beside the kernel's static arrays
+
 struct Engine {
   std::vector<fdtd_sim*> sims;
-  KernelConfig cfg;
+  KernelConfig asked;      // as set by the caller (may leave the choice to the autotuner)
+  KernelConfig cfg;        // the kernel in use
   StreamClass scls;        // streaming kernel
+  ResidentClass res;       // resident kernel
   DevBuf<SimDev> d_sims;   // plain kernel
   DevBuf<int4> d_tiles;    // plain kernel
   DevBuf<int> d_err;
@@ -520,6 +545,7 @@ struct Engine {
 
   void build_tiles() {
     reset_graph();
+    cfg = asked;
     int dev = 0, n_sm = 148;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
@@ -527,11 +553,12 @@ struct Engine {
       d_err.alloc(1);
       CK(cudaMemset(d_err.p, 0, sizeof(int)));
     }
-    if (cfg.variant == 1) {
-      if (cfg.ty == 0)
-        autotune(n_sm);
-      else
-        build_stream_tiles(n_sm);
+    if (cfg.variant == 1 && cfg.ty == 0) {
+      autotune(n_sm);
+      return;
+    }
+    if (cfg.variant != 0) {
+      build_shape(n_sm);
       return;
     }
     // plain kernel: 31 x 7 tiles, z cut into chunks
@@ -571,74 +598,237 @@ struct Engine {
     return tiles;
   }
 
-  // Picks the streaming kernel's (tile height, plane slots, z chunk) for this
-  // set of grids: each candidate runs a few time steps on the simulations
-  // themselves (their fields are cleared again by the next run), the fastest
-  // is kept and remembered for the same grid sizes.
+  // Tiles of the streaming kernel, or bricks of the resident one.
+  void build_shape(int n_sm) {
+    res.reset();
+    scls.reset();
+    if (cfg.variant == 2)
+      build_resident(n_sm);
+    else
+      build_stream_tiles(n_sm);
+  }
+
+  // Whether the resident kernel may step these simulations at all: one grid,
+  // nothing to do between two of its steps.
+  bool resident_allowed() const {
+    return sims.size() == 1 && sims[0]->monitors.empty() && sims[0]->adj_mode == 0;
+  }
+
+  // Partitions (bricks along x, y, z) worth timing, the cheapest first per
+  // number of blocks: the largest brick's cells and face cells bound a step.
+  // None when the grid's fields alone exceed the shared memory.
+  std::vector<std::array<int, 3>> resident_partitions(int n_sm) const {
+    std::vector<std::array<int, 3>> out;
+    const fdtd_sim* s = sims[0];
+    for (const int most : {n_sm, n_sm / 2, 32, 8}) {
+      double best = 1e300;
+      std::array<int, 3> pick{0, 0, 0};
+      for (int px = 1; px <= std::min(most, s->nx); ++px)
+        for (int py = 1; px * py <= most && py <= s->ny; ++py)
+          for (int pz = 1; px * py * pz <= most && pz <= s->nz; ++pz) {
+            const int bx = (s->nx + px - 1) / px, by = (s->ny + py - 1) / py, bz = (s->nz + pz - 1) / pz;
+            if (res_smem(bx, by, bz, 0) > kResSmemMax) continue;
+            const double cost = double(bx) * by * bz + 0.75 * (double(bx) * by + double(bx) * bz + double(by) * bz);
+            if (cost < best) {
+              best = cost;
+              pick = {px, py, pz};
+            }
+          }
+      if (pick[0] && std::find(out.begin(), out.end(), pick) == out.end()) out.push_back(pick);
+    }
+    return out;
+  }
+
+  // The resident kernel's lists and launch shape for cfg's partition; a size
+  // limit error when the bricks do not fit.
+  void build_resident(int n_sm) {
+    ResidentClass& c = res;
+    fdtd_sim* s = sims[0];
+    const int px = cfg.ty, py = cfg.stages, pz = cfg.zchunk, nb = px * py * pz;
+    if (nb > n_sm) throw ArgError{FDTD_ERR_LIMIT, "More bricks than SMs."};
+    const int bx = (s->nx + px - 1) / px, by = (s->ny + py - 1) / py, bz = (s->nz + pz - 1) / pz;
+    const int cells = bx * by * bz, nf = 2 * (by * bz + bx * bz + bx * by);
+    if (ResBox{0, 0, 0, bx, by, bz, 0, 0, 0}.size() * int64_t(3) >= kResNone || res_smem(bx, by, bz, 0) > kResSmemMax)
+      throw ArgError{FDTD_ERR_LIMIT, "Bricks do not fit in shared memory."};
+    const int n_rows = int(s->grid.rows.size());
+    c.count.alloc(size_t(nb));
+    DevBuf<int> map, nums, n_nums;
+    map.alloc(size_t(nb) * n_rows);
+    nums.alloc(size_t(nb) * kResScratch * cells);
+    n_nums.alloc(size_t(nb));
+    const ResScratch scratch{map.p, nums.p, n_rows, cells};
+    CK(cudaMemset(map.p, 0xff, map.n * sizeof(int)));
+    res_count_kernel<<<nb, 32>>>(s->dev, px, py, pz, scratch, c.count.p, n_nums.p);
+    CK(cudaGetLastError());
+    std::vector<int4> cnt(static_cast<size_t>(nb));
+    CK(cudaMemcpy(cnt.data(), c.count.p, cnt.size() * sizeof(int4), cudaMemcpyDeviceToHost));
+    int pairs = 0, local = 0;
+    for (const auto& k : cnt) {
+      pairs = std::max(pairs, k.z);
+      local = std::max(local, k.w);
+    }
+    const uint32_t state = res_smem(bx, by, bz, pairs);
+    if (state > kResSmemMax) throw ArgError{FDTD_ERR_LIMIT, "Bricks do not fit in shared memory."};
+    const int row_cap = std::min<int>(local, int((kResSmemMax - state) / kResRowBytes));
+    c.smem = state + uint32_t(row_cap) * kResRowBytes;
+    const size_t nl = size_t(nb) * cells;
+    c.lists.alloc(4 * nl);
+    c.row_ids.alloc(std::max<size_t>(1, size_t(nb) * row_cap));
+    c.stride.alloc(size_t(nb) * 64);
+    c.face.alloc(size_t(2) * nb * nf);
+    ResGrid& g = c.g;
+    g.s = s->dev;
+    g.px = px; g.py = py; g.pz = pz;
+    g.cap = cells;
+    g.row_cap = row_cap;
+    g.e_list = c.lists.p;
+    g.h_list = c.lists.p + nl;
+    g.e_words = c.lists.p + 2 * nl;
+    g.h_words = c.lists.p + 3 * nl;
+    g.count = c.count.p;
+    g.row_ids = c.row_ids.p;
+    g.stride = c.stride.p;
+    g.e_face = c.face.p;
+    g.h_face = c.face.p + size_t(nb) * nf;
+    g.face_cap = nf;
+    g.err = d_err.p;
+    res_build_kernel<<<nb, 32>>>(s->dev, px, py, pz, scratch, n_nums.p, cells, row_cap, c.lists.p, c.lists.p + nl,
+                                 c.lists.p + 2 * nl, c.lists.p + 3 * nl, c.row_ids.p, c.stride.p);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(0));
+    // every thread the same number of cells, and room for the face values
+    const int rounds = (cells + kResThreads - 1) / kResThreads;
+    c.threads = std::max({64, ((cells + rounds - 1) / rounds + 31) / 32 * 32, ((nf + 3) / 4 + 31) / 32 * 32});
+    if (c.threads > kResThreads) throw ArgError{FDTD_ERR_LIMIT, "Bricks have too many faces."};
+    c.faces = (nf + c.threads - 1) / c.threads;
+    c.blocks = nb;
+    const void* fn = resident_fn();
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kResSmemMax)));
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, c.threads, c.smem));
+    if (per_sm < 1) throw ArgError{FDTD_ERR_LIMIT, "Resident kernel does not fit on an SM."};
+    n_tiles = grid = nb;
+    zchunk_used = pz;
+  }
+
+  const void* resident_fn() const {
+    const bool small = res.threads <= 640;
+    return res.faces <= 1   ? small ? reinterpret_cast<const void*>(&res_step_kernel<1, 640>)
+                                    : reinterpret_cast<const void*>(&res_step_kernel<1, 1024>)
+           : res.faces <= 2 ? small ? reinterpret_cast<const void*>(&res_step_kernel<2, 640>)
+                                    : reinterpret_cast<const void*>(&res_step_kernel<2, 1024>)
+           : small          ? reinterpret_cast<const void*>(&res_step_kernel<4, 640>)
+                            : reinterpret_cast<const void*>(&res_step_kernel<4, 1024>);
+  }
+
+  // Steps n0 .. n1-1 by the resident kernel; the face words are cleared before
+  // a run's first launch (their tags are step numbers).
+  void launch_resident(cudaStream_t st, int n0, int n1) {
+    if (n0 == 0) CK(cudaMemsetAsync(res.face.p, 0, res.face.n * sizeof(unsigned long long), st));
+    res.g.s = sims[0]->dev;
+    res.g.wait_limit = wait_limit;
+    void* args[] = {&res.g, &n0, &n1};
+    CK(cudaLaunchCooperativeKernel(resident_fn(), dim3(unsigned(res.blocks)), dim3(unsigned(res.threads)), args,
+                                   res.smem, st));
+  }
+
+  // Time buffer that holds the state before step n.
+  int state_buf(int n) const { return cfg.variant == 2 ? 0 : n & 1; }
+
+  // Picks the step kernel and its shape for this set of grids: each candidate
+  // runs a few time steps on the simulations themselves (their fields are
+  // cleared again by the next run), the fastest is kept and remembered for the
+  // same grid sizes. A grid whose state fits in shared memory takes the
+  // resident kernel, whose partitions are timed (from 24x20x16 to 120x110x80
+  // cells it takes a third to three quarters of the streaming kernels' time per
+  // step, the least gain at the largest that fits); the others the streaming
+  // one.
   void autotune(int n_sm) {
     tune_ms = 0;
     tune_trials = 0;
-    std::vector<int> key;
+    if (resident_allowed()) {
+      std::vector<TuneChoice> cand;
+      for (const auto& p : resident_partitions(n_sm)) cand.push_back({2, p[0], p[1], p[2], 0});
+      if (!cand.empty() && tune(n_sm, cand, 2)) return;
+    }
+    std::vector<TuneChoice> cand;
+    for (const auto& c : kTuneCandidates) cand.push_back({c[0], c[1], c[2], c[3], c[4]});
+    tune(n_sm, cand, 1);
+  }
+
+  // Times the candidates (all of one kernel) and builds the best one; false
+  // when none fits.
+  bool tune(int n_sm, const std::vector<TuneChoice>& cand, int variant) {
+    std::vector<int> key{variant};
     int nt_min = 1 << 30;
     for (auto* s : sims) {
       key.insert(key.end(), {s->nx, s->ny, s->nz});
       nt_min = std::min(nt_min, s->prepared_nt);
     }
-    auto apply = [&](const TuneChoice& c) {
+    const KernelConfig auto_cfg = cfg;
+    auto build = [&](const TuneChoice& c) -> bool {
       cfg.variant = c[0];
       cfg.ty = c[1];
       cfg.stages = c[2];
       cfg.zchunk = c[3];
       cfg.one_list = c[4];
+      try {
+        build_shape(n_sm);
+      } catch (const ArgError& e) {
+        cfg = auto_cfg;
+        if (e.code != FDTD_ERR_LIMIT) throw;
+        return false;  // this shape does not fit these grids
+      }
+      return true;
     };
+    bool cached = false;
+    TuneChoice best{};
     {
       std::lock_guard<std::mutex> lock(g_tune_mutex);
       auto it = g_tune_cache.find(key);
       if (it != g_tune_cache.end()) {
-        apply(it->second);
-        build_stream_tiles(n_sm);
-        return;
+        cached = true;
+        best = it->second;
       }
     }
-    const int warm = 2, timed = std::min(8, nt_min - warm);
-    TuneChoice best = {kTuneCandidates[0][0], kTuneCandidates[0][1], kTuneCandidates[0][2],
-                       kTuneCandidates[0][3], kTuneCandidates[0][4]};
-    if (timed >= 2) {
-      const auto t0 = std::chrono::steady_clock::now();
-      init();
-      cudaStream_t st = stream();
-      float best_ms = 1e30f;
-      for (const auto& cand : kTuneCandidates) {
-        apply({cand[0], cand[1], cand[2], cand[3], cand[4]});
-        try {
-          build_stream_tiles(n_sm);
-        } catch (const ArgError& e) {
-          if (e.code != FDTD_ERR_LIMIT) throw;
-          continue;  // this shape's slots do not fit next to these grids' split slots
-        }
-        CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), st));
-        for (int n = 0; n < warm; ++n) launch_step(st, n);
-        CK(cudaEventRecord(ev0, st));
-        for (int n = warm; n < warm + timed; ++n) launch_step(st, n);
-        CK(cudaEventRecord(ev1, st));
-        CK(cudaStreamSynchronize(st));
-        float ms = 0;
-        CK(cudaEventElapsedTime(&ms, ev0, ev1));
-        ++tune_trials;
-        if (ms < best_ms) {
-          best_ms = ms;
-          best = {cand[0], cand[1], cand[2], cand[3], cand[4]};
-        }
-      }
-      check_error();
-      tune_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (cached && build(best)) return true;  // (a model of the same size may hold more split cells)
+    // (a launch of the resident kernel also loads and stores the state)
+    const int warm = 2, timed = std::min(variant == 2 ? 64 : 8, nt_min - warm);
+    bool found = false;
+    if (timed < 2) {
+      for (const auto& c : cand)
+        if (build(c)) return true;
+      return false;
     }
+    const auto t0 = std::chrono::steady_clock::now();
+    init();
+    cudaStream_t st = stream();
+    float best_ms = 1e30f;
+    for (const auto& c : cand) {
+      if (!build(c)) continue;
+      if (scls.d_counter.n) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), st));
+      launch_steps(st, 0, warm);
+      CK(cudaEventRecord(ev0, st));
+      launch_steps(st, warm, warm + timed);
+      CK(cudaEventRecord(ev1, st));
+      CK(cudaStreamSynchronize(st));
+      float ms = 0;
+      CK(cudaEventElapsedTime(&ms, ev0, ev1));
+      ++tune_trials;
+      if (ms < best_ms) {
+        best_ms = ms;
+        best = c;
+        found = true;
+      }
+    }
+    check_error();
+    tune_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (!found) return false;
     {
       std::lock_guard<std::mutex> lock(g_tune_mutex);
       g_tune_cache[key] = best;
     }
-    apply(best);
-    build_stream_tiles(n_sm);
+    return build(best);
   }
 
   // Streaming kernel: 31 x TY column tiles cut in z chunks of at most 62
@@ -646,7 +836,6 @@ struct Engine {
   // planes that hold split-field cells.
   void build_stream_tiles(int n_sm) {
     StreamClass& c = scls;
-    c.reset();
     const void* fn = nullptr;
     int threads = 0, smem = 0, ty = 0;
     {
@@ -825,10 +1014,25 @@ struct Engine {
     return int(c.n_tiles > 0) + int(c.n_tiles_p > 0);
   }
 
+  // Time steps n0 .. n1-1 on st; returns how many launches that took, a launch
+  // of the resident kernel counted once per step.
+  int launch_steps(cudaStream_t st, int n0, int n1) {
+    if (cfg.variant == 2) {
+      launch_resident(st, n0, n1);
+      return n1 - n0;
+    }
+    int k = 0;
+    for (int n = n0; n < n1; ++n) k += launch_step(st, n);
+    return k;
+  }
+
   // The kernels of time step n on st; returns how many were launched.
   int launch_step(cudaStream_t st, int n) {
     if (cfg.variant == 1) {
       return launch_stream_step(st, n, 0, 1 << 30, true);
+    } else if (cfg.variant == 2) {
+      launch_resident(st, n, n + 1);
+      return 1;
     } else {
       fdtd_step_kernel<kTileY><<<n_tiles, dim3(32, kBlockY), 0, st>>>(d_sims.p, d_tiles.p, n);
       CK(cudaGetLastError());
@@ -1297,7 +1501,32 @@ struct Engine {
     }
     if (scls.d_counter.n) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), st));
     int dft_from = 0;
-    for (int n = 0; n < nt; ++n) {
+    auto dft_upto = [&](int n) {  // the DFT of steps dft_from .. n-1, in chunks
+      while (dft_from < n) {
+        const int to = std::min(n, dft_from / kDftChunk * kDftChunk + kDftChunk);
+        for (auto* s : sims)
+          if (s->n_series > 0 && s->n_freq > 0) {
+            DftDev d{s->n_series, s->n_freq, nt, s->d_series_start.p, s->d_term_probe.p, s->d_term_weight.p,
+                     s->d_omega.p, s->rec.p, s->dft_X.p};
+            dft_accumulate_kernel<<<dim3(s->n_freq, s->n_series), 256, 0, st>>>(d, dft_from, to);
+            CK(cudaGetLastError());
+            ++dft_launches;
+          }
+        dft_from = to;
+      }
+    };
+    if (cfg.variant == 2) {
+      // nothing to do between the steps of a launch (one step per launch when
+      // every launch is asked to come from the host)
+      const int most = use_graph ? kResidentSteps : 1;
+      for (int n = 0; n < nt;) {
+        const int to = std::min(nt, n + most);
+        step_launches += launch_steps(st, n, to);
+        n = to;
+        if (n % kDftChunk == 0 || n == nt) dft_upto(n);
+      }
+    }
+    for (int n = 0; n < nt && cfg.variant != 2; ++n) {
       for (auto* s : sims)
         if (s->ckpt_every > 0 && n % s->ckpt_every == 0 && s->ckpt.n) {
           const size_t N = s->cells_padded, b = size_t(n & 1);
@@ -1324,17 +1553,7 @@ struct Engine {
           monitor_kernel<<<64, 256, 0, st>>>(s->d_dev.p, s->d_mons.p, int(s->monitors.size()), n, (n + 1) & 1);
           CK(cudaGetLastError());
         }
-      if ((n + 1) % kDftChunk == 0 || n + 1 == nt) {
-        for (auto* s : sims)
-          if (s->n_series > 0 && s->n_freq > 0) {
-            DftDev d{s->n_series, s->n_freq, nt, s->d_series_start.p, s->d_term_probe.p, s->d_term_weight.p,
-                     s->d_omega.p, s->rec.p, s->dft_X.p};
-            dft_accumulate_kernel<<<dim3(s->n_freq, s->n_series), 256, 0, st>>>(d, dft_from, n + 1);
-            CK(cudaGetLastError());
-            ++dft_launches;
-          }
-        dft_from = n + 1;
-      }
+      if ((n + 1) % kDftChunk == 0 || n + 1 == nt) dft_upto(n + 1);
     }
     // sentinel: a diverged run ends with non-finite records or fields
     for (auto* s : sims) {
@@ -1344,7 +1563,7 @@ struct Engine {
                                                                                               d_err.p);
         CK(cudaGetLastError());
       }
-      const size_t b = size_t(nt & 1) * 6 * s->cells_padded;  // buffer the last step wrote
+      const size_t b = size_t(state_buf(nt)) * 6 * s->cells_padded;  // buffer the last step wrote
       nonfinite_check_kernel<<<296, 256, 0, st>>>(s->fields.p + b, int64_t(6 * s->cells_padded), d_err.p);
       CK(cudaGetLastError());
     }
@@ -1653,7 +1872,7 @@ void new_engine(fdtd_sim* s) {
   s->engine.reset();
   s->engine = std::make_unique<Engine>();
   s->engine->sims = {s};
-  s->engine->cfg = s->cfg;
+  s->engine->asked = s->cfg;
   s->engine->ext_stream = s->ext_stream;
   s->engine->use_graph = s->use_graph;
   s->engine->wait_limit = s->dbg_wait_limit;
@@ -2206,7 +2425,7 @@ int fdtd_batch_create(fdtd_sim* const* sims, int n_sims, fdtd_batch** out) {
     b->sims.push_back(sims[i]);
   }
   b->engine.sims = b->sims;
-  b->engine.cfg = default_config();
+  b->engine.asked = default_config();
   *out = b;
   return FDTD_OK;
 }
@@ -2218,11 +2437,11 @@ int fdtd_batch_set_kernel(fdtd_batch* b, int variant, int tile_y, int stages, in
       throw ArgError{FDTD_ERR_ARG, "variant must be 0 (plain) or 1 (stream)"};
     if (!kernel_exists(variant, tile_y, stages))
       throw ArgError{FDTD_ERR_ARG, "No kernel instantiated for this variant / tile height / stage count."};
-    b->engine.cfg.variant = variant;
-    b->engine.cfg.ty = tile_y;
-    b->engine.cfg.stages = stages;
-    b->engine.cfg.zchunk = zchunk;
-    b->engine.cfg.one_list = one_list_env();
+    b->engine.asked.variant = variant;
+    b->engine.asked.ty = tile_y;
+    b->engine.asked.stages = stages;
+    b->engine.asked.zchunk = zchunk;
+    b->engine.asked.one_list = one_list_env();
     b->dirty = true;
   });
 }
