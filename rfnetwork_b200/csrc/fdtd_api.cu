@@ -450,6 +450,8 @@ struct ResidentClass {
   DevBuf<int4> count;
   DevBuf<uint16_t> stride, row_ids;
   DevBuf<unsigned long long> face;   // E faces, then H faces
+  DevBuf<uint2> mon_list;
+  DevBuf<int> mon_count;
   void reset() {
     blocks = 0;
     lists.free();
@@ -457,6 +459,8 @@ struct ResidentClass {
     stride.free();
     row_ids.free();
     face.free();
+    mon_list.free();
+    mon_count.free();
   }
 };
 
@@ -483,6 +487,8 @@ struct Engine {
   cudaEvent_t cap_fork = nullptr, cap_join = nullptr;
   cudaStream_t step_side = nullptr;                    // the plain-tile kernel beside the general one
   cudaEvent_t step_fork = nullptr, step_join = nullptr;
+  cudaStream_t mon_stream = nullptr;                   // plane monitors beside the next step
+  cudaEvent_t mon_fork = nullptr, mon_join = nullptr;
   cudaStream_t rep_stream = nullptr;                   // checkpointed adjoint: segment replays
   cudaEvent_t seg_done[2] = {nullptr, nullptr};        // replay of a segment into history half k & 1 done
   cudaEvent_t seg_free[2] = {nullptr, nullptr};        // its reversal done: the half may be refilled
@@ -511,6 +517,9 @@ struct Engine {
       CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
       CK(cudaStreamCreateWithPriority(&rep_stream, cudaStreamNonBlocking, hi));
     }
+    if (!mon_stream) CK(cudaStreamCreateWithFlags(&mon_stream, cudaStreamNonBlocking));
+    if (!mon_fork) CK(cudaEventCreateWithFlags(&mon_fork, cudaEventDisableTiming));
+    if (!mon_join) CK(cudaEventCreateWithFlags(&mon_join, cudaEventDisableTiming));
     if (!step_side) CK(cudaStreamCreateWithFlags(&step_side, cudaStreamNonBlocking));
     if (!step_fork) CK(cudaEventCreateWithFlags(&step_fork, cudaEventDisableTiming));
     if (!step_join) CK(cudaEventCreateWithFlags(&step_join, cudaEventDisableTiming));
@@ -531,6 +540,9 @@ struct Engine {
       if (seg_free[h]) cudaEventDestroy(seg_free[h]);
     }
     if (rep_stream) cudaStreamDestroy(rep_stream);
+    if (mon_fork) cudaEventDestroy(mon_fork);
+    if (mon_join) cudaEventDestroy(mon_join);
+    if (mon_stream) cudaStreamDestroy(mon_stream);
     if (step_fork) cudaEventDestroy(step_fork);
     if (step_join) cudaEventDestroy(step_join);
     if (step_side) cudaStreamDestroy(step_side);
@@ -611,7 +623,7 @@ struct Engine {
   // Whether the resident kernel may step these simulations at all: one grid,
   // nothing to do between two of its steps.
   bool resident_allowed() const {
-    return sims.size() == 1 && sims[0]->monitors.empty() && sims[0]->adj_mode == 0;
+    return sims.size() == 1 && sims[0]->adj_mode == 0;
   }
 
   // Partitions (bricks along x, y, z) worth timing, the cheapest first per
@@ -692,6 +704,26 @@ struct Engine {
     g.h_face = c.face.p + size_t(nb) * nf;
     g.face_cap = nf;
     g.err = d_err.p;
+    g.mons = s->d_mons.p;
+    g.n_mon = int(s->monitors.size());
+    if (g.n_mon > 0) {
+      std::vector<MonDev> mons;
+      for (const auto& m : s->monitors)
+        mons.push_back(MonDev{m.field, m.axis, m.position, m.n_step, m.n_freq, m.n1, m.n2, nullptr, nullptr});
+      int most_el = 1;
+      for (int b = 0; b < nb; ++b) {
+        int el = 0;
+        for (const auto& m : mons) el += res_mon_elements(m, res_box(s->dev, px, py, pz, b));
+        most_el = std::max(most_el, el);
+      }
+      c.mon_list.alloc(size_t(nb) * most_el);
+      c.mon_count.alloc(size_t(nb));
+      g.mon_cap = most_el;
+      g.mon_list = c.mon_list.p;
+      g.mon_count = c.mon_count.p;
+      res_monitor_kernel<<<nb, 128>>>(s->dev, px, py, pz, s->d_mons.p, g.n_mon, most_el, c.mon_list.p, c.mon_count.p);
+      CK(cudaGetLastError());
+    }
     res_build_kernel<<<nb, 32>>>(s->dev, px, py, pz, scratch, n_nums.p, cells, row_cap, c.lists.p, c.lists.p + nl,
                                  c.lists.p + 2 * nl, c.lists.p + 3 * nl, c.row_ids.p, c.stride.p);
     CK(cudaGetLastError());
@@ -1501,6 +1533,7 @@ struct Engine {
     }
     if (scls.d_counter.n) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), st));
     int dft_from = 0;
+    bool mon_pending = false;
     auto dft_upto = [&](int n) {  // the DFT of steps dft_from .. n-1, in chunks
       while (dft_from < n) {
         const int to = std::min(n, dft_from / kDftChunk * kDftChunk + kDftChunk);
@@ -1548,13 +1581,33 @@ struct Engine {
       }
       step_launches += launch_step(st, n);
       if (n_caps) CK(cudaStreamWaitEvent(st, cap_join, 0));
+      // The monitors of step n read the buffer that step n + 1 only reads: they
+      // run on a side stream beside it, and step n + 2, which overwrites that
+      // buffer, waits for them.
+      if (mon_pending) {
+        CK(cudaStreamWaitEvent(st, mon_join, 0));
+        mon_pending = false;
+      }
+      bool sample = false;
       for (auto* s : sims)
-        if (!s->monitors.empty()) {
-          monitor_kernel<<<64, 256, 0, st>>>(s->d_dev.p, s->d_mons.p, int(s->monitors.size()), n, (n + 1) & 1);
-          CK(cudaGetLastError());
-        }
+        for (const auto& m : s->monitors) sample = sample || monitor_samples(n, m.n_step);
+      if (sample) {
+        CK(cudaEventRecord(mon_fork, st));
+        CK(cudaStreamWaitEvent(mon_stream, mon_fork, 0));
+        for (auto* s : sims)
+          if (!s->monitors.empty()) {
+            int most = 1;
+            for (const auto& m : s->monitors) most = std::max(most, m.n1 * m.n2);
+            monitor_kernel<<<dim3(unsigned(std::min(64, (most + 127) / 128)), unsigned(s->monitors.size())), 128, 0,
+                             mon_stream>>>(s->d_dev.p, s->d_mons.p, n, (n + 1) & 1);
+            CK(cudaGetLastError());
+          }
+        CK(cudaEventRecord(mon_join, mon_stream));
+        mon_pending = true;
+      }
       if ((n + 1) % kDftChunk == 0 || n + 1 == nt) dft_upto(n + 1);
     }
+    if (mon_pending) CK(cudaStreamWaitEvent(st, mon_join, 0));
     // sentinel: a diverged run ends with non-finite records or fields
     for (auto* s : sims) {
       const int64_t nrec = int64_t(s->probes.size()) * nt;

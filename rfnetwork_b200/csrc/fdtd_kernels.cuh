@@ -462,53 +462,63 @@ struct MonDev {
   const float2* phase;       // [Nm][n_freq]
 };
 
+// Whether a monitor samples step n, and as which of its samples (solver.cpp:1129-1161).
+__host__ __device__ __forceinline__ bool monitor_samples(int n, int n_step) { return n == 0 || n % n_step == 0; }
+
+// One element of a monitor at sample mn: a time sample, or the running sums of
+// its phasors.
+__device__ __forceinline__ void monitor_add(const MonDev& M, int total, int e, int mn, float v) {
+  if (M.n_freq == 0) {
+    static_cast<float*>(M.out)[size_t(mn) * total + e] = v;
+    return;
+  }
+  float2* const o = static_cast<float2*>(M.out) + e;
+  const float2* const ph = M.phase + size_t(mn) * M.n_freq;
+  for (int f = 0; f < M.n_freq; ++f) {
+    const float2 p = __ldg(ph + f);
+    float2 acc = o[size_t(f) * total];
+    acc.x = __fmaf_rn(v, p.x, acc.x);
+    acc.y = __fmaf_rn(v, p.y, acc.y);
+    o[size_t(f) * total] = acc;
+  }
+}
+
 // Samples the fields after step n (E and H of the new buffer), i.e. after the
 // sources of the step are applied, as the CPU engine does (solver.cpp:1129-1161).
-__global__ void monitor_kernel(const SimDev* __restrict__ sim, const MonDev* __restrict__ mons, int n_mon, int n,
-                               int buf) {
+// One row of blocks per monitor: a plane's elements are a few thousand chains of
+// dependent loads, so a far-field box's 36 planes go side by side (one after
+// the other they took 60 us per step on planes of 72x64 cells, five times the
+// step itself).
+__global__ void monitor_kernel(const SimDev* __restrict__ sim, const MonDev* __restrict__ mons, int n, int buf) {
   const SimDev& S = *sim;
-  for (int m = 0; m < n_mon; ++m) {
-    const MonDev M = mons[m];
-    if (n > 0 && (n % M.n_step) != 0) continue;
-    const int mn = n / M.n_step;
-    const int total = M.n1 * M.n2;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-      const int a = e / M.n2, b = e % M.n2;
-      int x, y, z;
-      if (M.axis == 0) { x = M.position; y = a; z = b; }
-      else if (M.axis == 1) { x = a; y = M.position; z = b; }
-      else { x = a; y = b; z = M.position; }
-      if (x < 0 || y < 0 || z < 0 || x >= S.nx || y >= S.ny || z >= S.nz) continue;
-      const int idx = z * S.plane + y * S.pitch + x;
+  const MonDev M = mons[blockIdx.y];
+  if (!monitor_samples(n, M.n_step)) return;
+  const int mn = n / M.n_step;
+  const int total = M.n1 * M.n2;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
+    const int a = e / M.n2, b = e % M.n2;
+    int x, y, z;
+    if (M.axis == 0) { x = M.position; y = a; z = b; }
+    else if (M.axis == 1) { x = a; y = M.position; z = b; }
+    else { x = a; y = b; z = M.position; }
+    if (x < 0 || y < 0 || z < 0 || x >= S.nx || y >= S.ny || z >= S.nz) continue;
+    const int idx = z * S.plane + y * S.pitch + x;
+    float v;
+    if (M.field < 3) {
       const float4 r7 = S.rows[8 * S.mat[idx] + 7];
-      const uint32_t flags = __float_as_uint(r7.z);
-      float v;
-      if (M.field < 3) {
-        if (flags & (kCompSplit0 << M.field)) {
-          int cs;
-          const float2* pp = split_ptr(S.sp, buf, split_store(S.sp, S.nx, S.ny, S.nz, x, y, z), x, y, z,
-                                       __float_as_int(r7.w), cs);
-          const float2 p = pp[M.field * cs];
-          v = p.x + p.y;
-        } else {
-          v = S.E[buf][M.field][idx];
-        }
+      if (__float_as_uint(r7.z) & (kCompSplit0 << M.field)) {
+        int cs;
+        const float2* pp = split_ptr(S.sp, buf, split_store(S.sp, S.nx, S.ny, S.nz, x, y, z), x, y, z,
+                                     __float_as_int(r7.w), cs);
+        const float2 p = pp[M.field * cs];
+        v = p.x + p.y;
       } else {
-        v = S.H[buf][M.field - 3][idx];
+        v = S.E[buf][M.field][idx];
       }
-      if (M.n_freq == 0) {
-        static_cast<float*>(M.out)[size_t(mn) * total + e] = v;
-      } else {
-        float2* o = static_cast<float2*>(M.out);
-        for (int f = 0; f < M.n_freq; ++f) {
-          const float2 ph = M.phase[size_t(mn) * M.n_freq + f];
-          float2 acc = o[size_t(f) * total + e];
-          acc.x += v * ph.x;
-          acc.y += v * ph.y;
-          o[size_t(f) * total + e] = acc;
-        }
-      }
+    } else {
+      v = S.H[buf][M.field - 3][idx];
     }
+    monitor_add(M, total, e, mn, v);
   }
 }
 

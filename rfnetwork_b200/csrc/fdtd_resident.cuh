@@ -25,6 +25,9 @@
 //             round trip. A word is written again only after its reader has
 //             answered with its own faces of the same step, so one buffer is
 //             enough
+//   monitors  a plane monitor's elements in a brick are a list of the brick
+//             (res_monitor_kernel); after a sampled step one more barrier, then
+//             every thread adds its elements, sums kept in global memory
 //   waits     every poll is bounded; a block whose poll expires votes at the
 //             next barrier, records an error code and returns
 //
@@ -106,6 +109,10 @@ struct ResGrid {
   unsigned long long* e_face;  // [brick][face_cap] (value, tag)
   unsigned long long* h_face;
   int face_cap;
+  const MonDev* mons;      // plane monitors
+  int n_mon, mon_cap;
+  const uint2* mon_list;   // [brick][mon_cap]: field word | monitor << 16 | H side << 31, element
+  const int* mon_count;    // per brick
   int* err;
   uint32_t wait_limit;
 };
@@ -122,7 +129,7 @@ struct ResBox {
   __host__ __device__ int size() const { return sz() * (bz + 1); }
 };
 
-__device__ __forceinline__ ResBox res_box(const SimDev& S, int px, int py, int pz, int b) {
+__host__ __device__ __forceinline__ ResBox res_box(const SimDev& S, int px, int py, int pz, int b) {
   ResBox r;
   r.ix = b % px;
   r.iy = (b / px) % py;
@@ -375,6 +382,41 @@ res_build_kernel(const SimDev s, int px, int py, int pz, const ResScratch X, con
     }
     __syncwarp();
   }
+}
+
+// The part of [0, n) of a monitor's in-plane axis, or its position, that lies
+// in a brick's [c0, c0 + cn).
+__host__ __device__ __forceinline__ int res_mon_elements(const MonDev& M, const ResBox& r) {
+  const int lo[3] = {r.x0, r.y0, r.z0}, n[3] = {r.bx, r.by, r.bz};
+  if (M.position < lo[M.axis] || M.position >= lo[M.axis] + n[M.axis]) return 0;
+  return n[M.axis == 0 ? 1 : 0] * n[M.axis == 2 ? 1 : 2];
+}
+
+// Lists the monitor elements of one brick (one block), monitor by monitor, in
+// the order of the monitor's output.
+__global__ void __launch_bounds__(128)
+res_monitor_kernel(const SimDev s, int px, int py, int pz, const MonDev* __restrict__ mons, int n_mon, int cap,
+                   uint2* __restrict__ list, int* __restrict__ count) {
+  const ResBox r = res_box(s, px, py, pz, blockIdx.x);
+  const int e0 = 1 + r.sy() + r.sz();
+  int base = 0;
+  for (int m = 0; m < n_mon; ++m) {
+    const MonDev M = mons[m];
+    const int n = res_mon_elements(M, r), n2 = M.axis == 2 ? r.by : r.bz;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const int a = i / n2, b = i - a * n2;
+      const int lx = M.axis == 0 ? M.position - r.x0 : a;
+      const int ly = M.axis == 0 ? a : M.axis == 1 ? M.position - r.y0 : b;
+      const int lz = M.axis == 2 ? M.position - r.z0 : b;
+      const int k = lz * r.sz() + ly * r.sy() + lx;
+      const int ga = M.axis == 0 ? r.y0 + ly : r.x0 + lx, gb = M.axis == 2 ? r.y0 + ly : r.z0 + lz;
+      const uint32_t word = M.field < 3 ? uint32_t(3 * (k + e0) + M.field) : uint32_t(3 * k + M.field - 3);
+      list[size_t(blockIdx.x) * cap + base + i] =
+          make_uint2(word | uint32_t(m) << 16 | (M.field < 3 ? 0u : 1u << 31), uint32_t(ga * M.n2 + gb));
+    }
+    base += n;
+  }
+  if (threadIdx.x == 0) count[blockIdx.x] = base;
 }
 
 // Shared bytes of a brick: its local rows (12 E words, 12 H words: Da, Db of
@@ -678,6 +720,22 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
       h[1] = vy;
       h[2] = vz;
       if (f & kResProbe) res_record(S, __ldg(rows + 8 * (d.x >> 16) + 7), n, false, vx, vy, vz);
+    }
+    if (G.n_mon > 0) {
+      bool any = false;
+      for (int m = 0; m < G.n_mon; ++m) any |= monitor_samples(n, G.mons[m].n_step);
+      if (any) {  // (the same for every thread)
+        __syncthreads();
+        const uint2* const ml = G.mon_list + size_t(blockIdx.x) * G.mon_cap;
+        const int nm = G.mon_count[blockIdx.x];
+        for (int i = tid; i < nm; i += T) {
+          const uint2 d = __ldg(ml + i);
+          const MonDev M = G.mons[(d.x >> 16) & 0x7fffu];
+          if (!monitor_samples(n, M.n_step)) continue;
+          const float v = ((d.x >> 31) ? H : E)[d.x & 0xffffu];
+          monitor_add(M, M.n1 * M.n2, int(d.y), n / M.n_step, v);
+        }
+      }
     }
   }
   __syncthreads();

@@ -115,3 +115,38 @@ def test_partition_follows_the_run(engine_lib):
     assert np.array_equal(sim.probe_values(), a) and np.array_equal(sim.dft(), X)
     batch.close()
     sim.close()
+
+
+# time samples and phasors, sampled every step and every third, on planes at the
+# grid's ends and inside, of split (layer) and unsplit cells
+@pytest.mark.parametrize("shape,n_pml", [((34, 30, 26), 4), ((3, 6, 4), 0)])
+def test_monitors_equal_plain(engine_lib, shape, n_pml):
+    nt = 50
+    phase = np.exp(-1j * 0.2 * np.arange(nt + 1)[:, None] * np.arange(1, 4)[None]).astype(np.complex64)
+
+    def make():
+        if n_pml:
+            sim, _ = _model_sim(configs.microstrip(n=shape, n_pml=n_pml, nt=nt))
+        else:
+            sim = _random_sim(shape, 8, nt, 1, tile_y=0)
+        for axis in range(3):
+            for field in range(6):
+                for k, pos in enumerate((1, shape[axis] // 2, shape[axis] - 1)):
+                    if (field + k) % 2:
+                        sim.add_monitor(field, axis, pos, 1 + 2 * (k == 1), phase=phase)
+                    elif k == 1:
+                        sim.add_monitor(field, axis, pos, 3)
+        return sim
+
+    out = []
+    for plain in (False, True):
+        sim = make()
+        if plain:
+            sim.set_kernel(0)
+        sim.run(nt)
+        assert plain or sim.stats()["variant"] == 2
+        out.append([sim.monitor(m) for m in range(len(sim.monitors))])
+        sim.close()
+    assert any(np.abs(b).max() > 0 for b in out[1])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
