@@ -2719,53 +2719,74 @@ int fdtd_nf2ff(const fdtd_nf2ff_face* faces, int n_faces, int n_freq, const floa
       n_cells += int64_t(fc.n0) * fc.n1;
     }
     if (n_cells * n_freq > (int64_t(1) << 31)) throw ArgError{FDTD_ERR_LIMIT, "fdtd_nf2ff: surface too large"};
-    // cells of all faces, one block per frequency: position and ds J, ds M
-    std::vector<Nf2ffCell> host(size_t(std::max<int64_t>(1, n_cells * n_freq)));
-    int64_t c0 = 0;
+    // one block of device memory: the faces, then beta, theta, phi and the
+    // faces' arrays as they come, then the parts' sums and the result
+    const size_t n_dir = size_t(n_theta) * n_phi;
+    size_t at = (size_t(std::max(1, n_faces)) * sizeof(Nf2ffFaceDev) + 3) / 4;  // floats
+    const size_t o_beta = at, o_theta = o_beta + n_freq, o_phi = o_theta + n_theta;
+    at = o_phi + n_phi;
+    std::vector<Nf2ffFaceDev> fd(size_t(std::max(1, n_faces)), Nf2ffFaceDev{});
+    int64_t first = 0;
     for (int i = 0; i < n_faces; ++i) {
       const fdtd_nf2ff_face& fc = faces[i];
-      const int64_t nc = int64_t(fc.n0) * fc.n1;
-      for (int64_t c = 0; c < nc; ++c) {
-        float xyz[3];
-        const int o0 = fc.axis == 0 ? 1 : 0, o1 = fc.axis == 2 ? 1 : 2;
-        xyz[fc.axis] = fc.pos;
-        xyz[o0] = fc.r0[c];
-        xyz[o1] = fc.r1[c];
-        const float ds = fc.ds[c];
-        for (int f = 0; f < n_freq; ++f) {
-          float v[12];
-          for (int q = 0; q < 3; ++q)
-            for (int k = 0; k < 2; ++k) {
-              v[2 * q + k] = ds * fc.J[((size_t(q) * n_freq + f) * nc + c) * 2 + k];
-              v[6 + 2 * q + k] = ds * fc.M[((size_t(q) * n_freq + f) * nc + c) * 2 + k];
-            }
-          Nf2ffCell& cell = host[size_t(f) * n_cells + c0 + c];
-          cell.pos = make_float4(xyz[0], xyz[1], xyz[2], 0.f);
-          cell.j01 = make_float4(v[0], v[1], v[2], v[3]);
-          cell.j2m0 = make_float4(v[4], v[5], v[6], v[7]);
-          cell.m12 = make_float4(v[8], v[9], v[10], v[11]);
-        }
-      }
-      c0 += nc;
+      const size_t nc = size_t(fc.n0) * fc.n1;
+      Nf2ffFaceDev& d = fd[size_t(i)];
+      d.axis = fc.axis;
+      d.cells = int(nc);
+      d.first = int(first);
+      d.pos = fc.pos;
+      d.r0 = int64_t(at);
+      d.r1 = int64_t(at + nc);
+      d.ds = int64_t(at + 2 * nc);
+      d.J = int64_t(at + 3 * nc);
+      d.M = d.J + int64_t(6 * n_freq * nc);
+      at = size_t(d.M) + 6 * n_freq * nc;
+      first += int64_t(nc);
     }
-    DevBuf<Nf2ffCell> d_cells;
-    DevBuf<float> d_beta, d_theta, d_phi;
-    DevBuf<float2> d_out;
-    d_cells.alloc(host.size());
-    CK(cudaMemcpy(d_cells.p, host.data(), host.size() * sizeof(Nf2ffCell), cudaMemcpyHostToDevice));
-    d_beta.alloc(size_t(n_freq));
-    CK(cudaMemcpy(d_beta.p, beta, size_t(n_freq) * 4, cudaMemcpyHostToDevice));
-    d_theta.alloc(size_t(n_theta));
-    CK(cudaMemcpy(d_theta.p, theta, size_t(n_theta) * 4, cudaMemcpyHostToDevice));
-    d_phi.alloc(size_t(n_phi));
-    CK(cudaMemcpy(d_phi.p, phi, size_t(n_phi) * 4, cudaMemcpyHostToDevice));
-    const size_t n_out = size_t(2) * n_freq * n_theta * n_phi;
-    d_out.alloc(n_out);
-    const dim3 grid(unsigned((int64_t(n_theta) * n_phi + kNf2ffThreads - 1) / kNf2ffThreads), unsigned(n_freq));
-    nf2ff_kernel<<<grid, kNf2ffThreads>>>(d_cells.p, int(n_cells), d_beta.p, d_theta.p, n_theta, d_phi.p, n_phi,
-                                          d_out.p);
+    const std::unique_ptr<float[]> host(new float[at]);  // every word is written below
+    std::memcpy(host.get(), fd.data(), fd.size() * sizeof(Nf2ffFaceDev));
+    std::memcpy(&host[o_beta], beta, size_t(n_freq) * 4);
+    std::memcpy(&host[o_theta], theta, size_t(n_theta) * 4);
+    std::memcpy(&host[o_phi], phi, size_t(n_phi) * 4);
+    for (int i = 0; i < n_faces; ++i) {
+      const fdtd_nf2ff_face& fc = faces[i];
+      const Nf2ffFaceDev& d = fd[size_t(i)];
+      const size_t nc = size_t(d.cells);
+      if (!nc) continue;
+      std::memcpy(&host[size_t(d.r0)], fc.r0, nc * 4);
+      std::memcpy(&host[size_t(d.r1)], fc.r1, nc * 4);
+      std::memcpy(&host[size_t(d.ds)], fc.ds, nc * 4);
+      std::memcpy(&host[size_t(d.J)], fc.J, 6 * n_freq * nc * 4);
+      std::memcpy(&host[size_t(d.M)], fc.M, 6 * n_freq * nc * 4);
+    }
+    // parts: about eight blocks per SM in all (148 SMs), at least one chunk of
+    // cells each, and at most 256 MB of sums
+    const int64_t dir_blocks = int64_t((n_dir + kNf2ffThreads - 1) / kNf2ffThreads);
+    int64_t parts = (int64_t(148) * 8 + dir_blocks * n_freq - 1) / (dir_blocks * n_freq);
+    parts = std::min(parts, (n_cells + kNf2ffThreads - 1) / kNf2ffThreads);
+    parts = std::min<int64_t>(parts, (int64_t(256) << 20) / int64_t(96 * n_dir * size_t(n_freq)));
+    parts = std::max<int64_t>(1, std::min<int64_t>(parts, 65535));
+    const int64_t per = std::max<int64_t>(1, (n_cells + parts - 1) / parts);
+    const size_t n_out = 2 * size_t(n_freq) * n_dir;
+    const size_t o_sums = (at + 3) / 4 * 4, o_out = o_sums + (parts > 1 ? size_t(parts) * n_freq * 12 * n_dir * 2 : 0);
+    DevBuf<float> buf;
+    buf.alloc(o_out + 2 * n_out);
+    CK(cudaMemcpy(buf.p, host.get(), at * 4, cudaMemcpyHostToDevice));
+    const float *d_beta = buf.p + o_beta, *d_theta = buf.p + o_theta, *d_phi = buf.p + o_phi;
+    double* const d_sums = reinterpret_cast<double*>(buf.p + o_sums);
+    float2* const d_out = reinterpret_cast<float2*>(buf.p + o_out);
+    nf2ff_kernel<<<dim3(unsigned(dir_blocks), unsigned(n_freq), unsigned(parts)), kNf2ffThreads>>>(
+        buf.p, reinterpret_cast<const Nf2ffFaceDev*>(buf.p), n_faces, int(n_cells), int(per), d_beta, d_theta, n_theta,
+        d_phi, n_phi, d_sums, d_out);
     CK(cudaGetLastError());
-    CK(cudaMemcpy(out, d_out.p, n_out * sizeof(float2), cudaMemcpyDeviceToHost));
+    if (parts > 1) {
+      nf2ff_field_kernel<<<dim3(unsigned((n_dir + kNf2ffThreads / kNf2ffGroups - 1) / (kNf2ffThreads / kNf2ffGroups)),
+                                unsigned(n_freq)),
+                           kNf2ffThreads>>>(
+          d_sums, int(parts), d_beta, d_theta, n_theta, d_phi, n_phi, d_out);
+      CK(cudaGetLastError());
+    }
+    CK(cudaMemcpy(out, d_out, n_out * sizeof(float2), cudaMemcpyDeviceToHost));
   });
 }
 
