@@ -41,6 +41,7 @@ constexpr int kDftChunk = 256;  // steps between DFT accumulation passes
 constexpr int kResidentSteps = 16 * kDftChunk;  // most steps of one launch of the resident kernel
 constexpr int kMaxProbes = 1 << 20;
 constexpr int kMaxMonitors = 50;  // MAX_MONITORS, rfnetwork/core/inc/solver.h:15
+static_assert(kMaxMonitors <= kResMonitors, "monitor table of the resident kernel");
 
 // error text of the calls without a handle, kept per calling thread
 thread_local std::string g_error;
@@ -464,7 +465,7 @@ struct ResidentClass {
   }
 };
 
-constexpr uint32_t kResSmemMax = 232448 - 1024;  // dynamic shared bytes beside the kernel's static arrays
+constexpr uint32_t kResSmemMax = 232448 - 4096;  // dynamic shared bytes beside the kernel's static arrays
 
 struct Engine {
   std::vector<fdtd_sim*> sims;
@@ -706,6 +707,7 @@ struct Engine {
     g.err = d_err.p;
     g.mons = s->d_mons.p;
     g.n_mon = int(s->monitors.size());
+    g.acc_f = g.acc_cap = 0;
     if (g.n_mon > 0) {
       std::vector<MonDev> mons;
       for (const auto& m : s->monitors)
@@ -720,6 +722,15 @@ struct Engine {
       c.mon_count.alloc(size_t(nb));
       g.mon_cap = most_el;
       g.mon_list = c.mon_list.p;
+      // sums in shared memory when every monitor is a phasor monitor of the same
+      // number of frequencies
+      bool uniform = mons[0].n_freq > 0;
+      for (const auto& m : mons) uniform = uniform && m.n_freq == mons[0].n_freq;
+      if (uniform) {
+        g.acc_f = mons[0].n_freq;
+        g.acc_cap = std::min<int>(most_el, int((kResSmemMax - c.smem) / (8u * uint32_t(g.acc_f))));
+        c.smem += uint32_t(g.acc_cap) * 8u * uint32_t(g.acc_f);
+      }
       g.mon_count = c.mon_count.p;
       res_monitor_kernel<<<nb, 128>>>(s->dev, px, py, pz, s->d_mons.p, g.n_mon, most_el, c.mon_list.p, c.mon_count.p);
       CK(cudaGetLastError());
@@ -743,15 +754,17 @@ struct Engine {
     zchunk_used = pz;
   }
 
-  const void* resident_fn() const {
-    const bool small = res.threads <= 640;
-    return res.faces <= 1   ? small ? reinterpret_cast<const void*>(&res_step_kernel<1, 640>)
-                                    : reinterpret_cast<const void*>(&res_step_kernel<1, 1024>)
-           : res.faces <= 2 ? small ? reinterpret_cast<const void*>(&res_step_kernel<2, 640>)
-                                    : reinterpret_cast<const void*>(&res_step_kernel<2, 1024>)
-           : small          ? reinterpret_cast<const void*>(&res_step_kernel<4, 640>)
-                            : reinterpret_cast<const void*>(&res_step_kernel<4, 1024>);
+  template <bool MON>
+  const void* resident_variant() const {
+    const bool small = res.threads <= 640;  // (more registers per thread)
+    return res.faces <= 1   ? small ? reinterpret_cast<const void*>(&res_step_kernel<1, 640, MON>)
+                                    : reinterpret_cast<const void*>(&res_step_kernel<1, 1024, MON>)
+           : res.faces <= 2 ? small ? reinterpret_cast<const void*>(&res_step_kernel<2, 640, MON>)
+                                    : reinterpret_cast<const void*>(&res_step_kernel<2, 1024, MON>)
+           : small          ? reinterpret_cast<const void*>(&res_step_kernel<4, 640, MON>)
+                            : reinterpret_cast<const void*>(&res_step_kernel<4, 1024, MON>);
   }
+  const void* resident_fn() const { return res.g.n_mon > 0 ? resident_variant<true>() : resident_variant<false>(); }
 
   // Steps n0 .. n1-1 by the resident kernel; the face words are cleared before
   // a run's first launch (their tags are step numbers).

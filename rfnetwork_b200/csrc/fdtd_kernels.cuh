@@ -474,12 +474,19 @@ __device__ __forceinline__ void monitor_add(const MonDev& M, int total, int e, i
   }
   float2* const o = static_cast<float2*>(M.out) + e;
   const float2* const ph = M.phase + size_t(mn) * M.n_freq;
-  for (int f = 0; f < M.n_freq; ++f) {
-    const float2 p = __ldg(ph + f);
-    float2 acc = o[size_t(f) * total];
-    acc.x = __fmaf_rn(v, p.x, acc.x);
-    acc.y = __fmaf_rn(v, p.y, acc.y);
-    o[size_t(f) * total] = acc;
+  for (int f0 = 0; f0 < M.n_freq; f0 += 4) {  // four sums in flight at a time
+    float2 acc[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (f0 + j < M.n_freq) acc[j] = o[size_t(f0 + j) * total];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (f0 + j < M.n_freq) {
+        const float2 p = __ldg(ph + f0 + j);
+        acc[j].x = __fmaf_rn(v, p.x, acc[j].x);
+        acc[j].y = __fmaf_rn(v, p.y, acc[j].y);
+        o[size_t(f0 + j) * total] = acc[j];
+      }
   }
 }
 

@@ -27,7 +27,10 @@
 //             enough
 //   monitors  a plane monitor's elements in a brick are a list of the brick
 //             (res_monitor_kernel); after a sampled step one more barrier, then
-//             every thread adds its elements, sums kept in global memory
+//             every thread adds its elements. The phasor sums stay in shared
+//             memory for the launch as far as they fit beside the rest (in
+//             global memory a 36-plane far-field box on 72x64x64 cells took 9 us
+//             per step, a chain of L2 round trips per element)
 //   waits     every poll is bounded; a block whose poll expires votes at the
 //             next barrier, records an error code and returns
 //
@@ -55,6 +58,7 @@ namespace rfn {
 
 constexpr int kResThreads = 1024;   // most threads of a block
 constexpr uint32_t kResNone = 0xffffu;
+constexpr int kResMonitors = 50;    // most plane monitors of a simulation
 // flags of a list entry beside the six bits of its split components
 constexpr uint32_t kResProbe = 1u << 6;   // the cell holds probes
 constexpr uint32_t kResGlobal = 1u << 7;  // its table row is read from global memory
@@ -113,6 +117,7 @@ struct ResGrid {
   int n_mon, mon_cap;
   const uint2* mon_list;   // [brick][mon_cap]: field word | monitor << 16 | H side << 31, element
   const int* mon_count;    // per brick
+  int acc_f, acc_cap;      // phasor sums in shared memory: frequencies, elements per brick (the first of its list)
   int* err;
   uint32_t wait_limit;
 };
@@ -438,12 +443,15 @@ __device__ __forceinline__ unsigned long long res_get(const unsigned long long* 
 }
 
 // Advances steps n0 .. n1-1 of the grid. FACES: face values of one side per
-// thread (at least a brick's face values / threads).
-template <int FACES, int THREADS>
+// thread (at least a brick's face values / threads). MON: with plane monitors.
+template <int FACES, int THREADS, bool MON>
 __global__ void __launch_bounds__(THREADS, 1)
 res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
-  extern __shared__ __align__(16) float4 s_rows[];  // E quads, H quads of the local rows, then fields, pairs
+  // E quads, H quads of the local rows, then fields, pairs, phasor sums
+  extern __shared__ __align__(16) float4 s_rows[];
   __shared__ int s_stride[64];
+  __shared__ MonDev s_mon[MON ? kResMonitors : 1];
+  __shared__ int s_sample[MON ? kResMonitors : 1];  // this step's sample of each monitor, -1: none
   const SimDev& S = G.s;
   const int T = blockDim.x, tid = threadIdx.x;
   const ResBox r = res_box(S, G.px, G.py, G.pz, blockIdx.x);
@@ -463,6 +471,19 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
   const uint2* const el = G.e_list + size_t(blockIdx.x) * G.cap;
   const uint2* const hl = G.h_list + size_t(blockIdx.x) * G.cap;
   const float4* const rows = S.rows;
+  // the monitor elements whose sums stay here: nm_in of the brick's nm, sum of
+  // frequency f of element i at acc[f * acc_cap + i]
+  float2* const acc = P + cnt.z;
+  const uint2* const ml = G.mon_list + size_t(blockIdx.x) * G.mon_cap;
+  const int nm = MON ? G.mon_count[blockIdx.x] : 0, nm_in = MON ? min(nm, G.acc_cap) : 0;
+  if (MON)
+    for (int m = tid; m < G.n_mon; m += T) s_mon[m] = G.mons[m];
+  for (int i = tid; i < nm_in; i += T) {
+    const uint2 d = ml[i];
+    const MonDev M = G.mons[(d.x >> 16) & 0x7fffu];
+    for (int f = 0; f < G.acc_f; ++f)
+      acc[f * G.acc_cap + i] = static_cast<const float2*>(M.out)[size_t(f) * M.n1 * M.n2 + d.y];
+  }
   for (int k = tid; k < 64; k += T) s_stride[k] = G.stride[size_t(blockIdx.x) * 64 + k];
   for (int k = tid; k < min(cnt.w, G.row_cap); k += T) {
     const float4* const row = rows + 8 * int(G.row_ids[size_t(blockIdx.x) * G.row_cap + k]);
@@ -721,26 +742,40 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
       h[2] = vz;
       if (f & kResProbe) res_record(S, __ldg(rows + 8 * (d.x >> 16) + 7), n, false, vx, vy, vz);
     }
-    if (G.n_mon > 0) {
-      bool any = false;
-      for (int m = 0; m < G.n_mon; ++m) any |= monitor_samples(n, G.mons[m].n_step);
-      if (any) {  // (the same for every thread)
-        __syncthreads();
-        const uint2* const ml = G.mon_list + size_t(blockIdx.x) * G.mon_cap;
-        const int nm = G.mon_count[blockIdx.x];
-        for (int i = tid; i < nm; i += T) {
-          const uint2 d = __ldg(ml + i);
-          const MonDev M = G.mons[(d.x >> 16) & 0x7fffu];
-          if (!monitor_samples(n, M.n_step)) continue;
-          const float v = ((d.x >> 31) ? H : E)[d.x & 0xffffu];
-          monitor_add(M, M.n1 * M.n2, int(d.y), n / M.n_step, v);
+    if (MON) {
+      for (int m = tid; m < G.n_mon; m += T)
+        s_sample[m] = monitor_samples(n, s_mon[m].n_step) ? n / s_mon[m].n_step : -1;
+      __syncthreads();
+      for (int i = tid; i < nm; i += T) {
+        const uint2 d = __ldg(ml + i);
+        const int m = int((d.x >> 16) & 0x7fffu), mn = s_sample[m];
+        if (mn < 0) continue;
+        const MonDev& M = s_mon[m];
+        const float v = ((d.x >> 31) ? H : E)[d.x & 0xffffu];
+        if (i < nm_in) {
+          const float2* const ph = M.phase + size_t(mn) * G.acc_f;
+          for (int f = 0; f < G.acc_f; ++f) {
+            const float2 p = __ldg(ph + f);
+            float2 a = acc[f * G.acc_cap + i];
+            a.x = __fmaf_rn(v, p.x, a.x);
+            a.y = __fmaf_rn(v, p.y, a.y);
+            acc[f * G.acc_cap + i] = a;
+          }
+        } else {
+          monitor_add(M, M.n1 * M.n2, int(d.y), mn, v);
         }
       }
     }
   }
   __syncthreads();
 
-  // ---- the state after the last step
+  // ---- the sums and the state after the last step
+  for (int i = tid; i < nm_in; i += T) {
+    const uint2 d = ml[i];
+    const MonDev M = G.mons[(d.x >> 16) & 0x7fffu];
+    for (int f = 0; f < G.acc_f; ++f)
+      static_cast<float2*>(M.out)[size_t(f) * M.n1 * M.n2 + d.y] = acc[f * G.acc_cap + i];
+  }
   for (int c = tid; c < cells; c += T) {
     const uint2 d = el[c];
     const uint32_t f = d.y >> 16;
