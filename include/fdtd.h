@@ -53,12 +53,13 @@ typedef struct fdtd_stats {
   int64_t h_split_cells; /* cells whose H components are stored as split fields */
   int n_tiles;           /* thread blocks per time step */
   int64_t step_launches; /* time-step kernel launches issued by the last run (a launch of the resident
-                            kernel advances many steps and counts once per step) */
+                            kernel advances many steps and counts once per step; the two half
+                            steps of a step count once) */
   int64_t dft_launches;  /* DFT kernel launches issued by the last run */
   double last_run_ms;    /* device time of the last run (CUDA events) */
   double compile_ms;     /* host time spent building the material table */
   int variant;           /* step kernel: 0 plain loads, 1 TMA streaming, 2 resident (tile_y, stages, zchunk:
-                            its bricks along x, y, z) */
+                            its bricks along x, y, z), 3 half steps (tile_y: threads per block) */
   int tile_y;            /* tile height (rows) of the step kernel */
   int stages;            /* shared-memory pipeline stages (TMA kernel) */
   int zchunk;            /* z planes per tile */
@@ -145,7 +146,9 @@ int fdtd_synchronize(fdtd_sim* s);
  * fastest, remembered per set of grid sizes for the life of the process. A
  * single grid whose state fits in the GPU's shared memory, without monitors
  * and without anything kept for a gradient, is then stepped by the resident
- * kernel (one cooperative launch for many steps; its partitions are timed). The
+ * kernel (one cooperative launch for many steps; its partitions are timed);
+ * for the others the half-step kernels (E, then H, in place) are candidates
+ * too, which RFN_FDTD_KERNEL=half asks for. The
  * default comes from RFN_FDTD_KERNEL (plain / stream) / RFN_FDTD_TY /
  * RFN_FDTD_STAGES / RFN_FDTD_ZCHUNK or is (1, 0, 6, 0): autotuned streaming.
  * RFN_FDTD_ONE_LIST=1 sends the plain tiles of an explicit streaming shape

@@ -58,6 +58,12 @@ struct AdjSim {
   const float* hist;         // forward history: [9][nb] per step = E_x E_y E_z, dA_x dB_x .. dB_z
 };
 
+// Place of cell (x, y, z) of a gradient box bnx x bny x bnz in its history and
+// gradient arrays: x fastest, as the warps that write and read them lie.
+__host__ __device__ __forceinline__ int64_t box_cell(int x, int y, int z, int bnx, int bny) {
+  return (int64_t(z) * bny + y) * bnx + x;
+}
+
 // Box history of one simulation at one step: E^n and the six H differences
 // the E update of step n uses.
 struct CapSim {
@@ -317,9 +323,8 @@ adj_step_kernel(const AdjSim* __restrict__ sims, const int4* __restrict__ tiles,
         wH[idx] = lh[0]; wH[N + idx] = lh[1]; wH[2 * N + idx] = lh[2];
       }
       if (A.hist && c >= A.bx0 && c < A.bx1 && r >= A.by0 && r < A.by1 && z >= A.bz0 && z < A.bz1) {
-        const int bny = A.by1 - A.by0, bnz = A.bz1 - A.bz0;
         const int64_t nb = A.nb;
-        const int64_t bi = (int64_t(c - A.bx0) * bny + (r - A.by0)) * bnz + (z - A.bz0);
+        const int64_t bi = box_cell(c - A.bx0, r - A.by0, z - A.bz0, A.bx1 - A.bx0, A.by1 - A.by0);
         const float* hs = A.hist + int64_t(n - hist_n0) * 9 * nb;
         adj_grad_cell(A.grad, nb, bi, hs, mu);
       }
@@ -369,15 +374,14 @@ __global__ void adj_inject_kernel(const AdjSim* __restrict__ sims, int step, int
 __global__ void adj_capture_kernel(const CapSim* __restrict__ caps, int n, int n0) {
   const CapSim& C = caps[blockIdx.y];
   const SimDev& s = C.s;
-  const int bnx = C.bx1 - C.bx0, bny = C.by1 - C.by0, bnz = C.bz1 - C.bz0;
-  (void)bnx;
+  const int bnx = C.bx1 - C.bx0, bny = C.by1 - C.by0;
   const int64_t nb = C.nb;
   float* hist = C.hist + int64_t(n - n0) * 9 * nb;
   const int b = n & 1;
   const float* const* E = s.E[b];
   const float* const* H = s.H[b];
   for (int64_t bi = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; bi < nb; bi += int64_t(gridDim.x) * blockDim.x) {
-    const int zz = int(bi % bnz), yy = int((bi / bnz) % bny), xx = int(bi / (int64_t(bnz) * bny));
+    const int xx = int(bi % bnx), yy = int((bi / bnx) % bny), zz = int(bi / (int64_t(bnx) * bny));
     const int x = C.bx0 + xx, y = C.by0 + yy, z = C.bz0 + zz;
     const int idx = z * s.plane + y * s.pitch + x;
     auto h = [&](int c, bool ok, int off) { return ok ? H[c][idx + off] : 0.f; };

@@ -347,8 +347,7 @@ adj_stream_kernel(const AdjSim* __restrict__ sims, const AdjMaps* __restrict__ m
           wH[idx] = lh[0]; wH[N + idx] = lh[1]; wH[2 * N + idx] = lh[2];
         }
         if (A.hist && c >= A.bx0 && c < A.bx1 && r >= A.by0 && r < A.by1 && z >= A.bz0 && z < A.bz1) {
-          const int bny = A.by1 - A.by0, bnz = A.bz1 - A.bz0;
-          const int64_t bi = (int64_t(c - A.bx0) * bny + (r - A.by0)) * bnz + (z - A.bz0);
+          const int64_t bi = box_cell(c - A.bx0, r - A.by0, z - A.bz0, A.bx1 - A.bx0, A.by1 - A.by0);
           adj_grad_cell(A.grad, A.nb, bi, A.hist + int64_t(n - hist_n0) * 9 * A.nb, mu);
         }
       }

@@ -29,6 +29,7 @@
 #include "fdtd_adjoint.cuh"
 #include "fdtd_nf2ff.cuh"
 #include "fdtd_step_stream.cuh"
+#include "fdtd_half.cuh"
 #include "fdtd_resident.cuh"
 #include "fdtd_adjoint_stream.cuh"
 #include <cudaTypedefs.h>
@@ -139,8 +140,9 @@ int threads_for_host() {
 // Kernel selection of an engine: the plain-load kernel (one cell per thread)
 // or the TMA-pipelined streaming kernel (tile height, plane slots), and the z chunk.
 struct KernelConfig {
-  int variant = 1;  // 0 plain loads, 1 TMA streaming, 2 resident (only ever the engine's own choice)
-  int ty = 0;       // tile height; 0 (with variant 1): autotuned (ty, stages, zchunk); resident: bricks along x
+  int variant = 1;  // 0 plain loads, 1 TMA streaming, 2 resident, 3 half steps (the engine's own choice)
+  int ty = 0;       // tile height; 0 (with variant 1): autotuned (ty, stages, zchunk); resident: bricks along x;
+                    // half steps: threads per block
   int stages = 6;   // streaming: shared-memory plane slots; resident: bricks along y
   int zchunk = 0;   // 0: pick from the grid size; resident: bricks along z
   int one_list = 0; // streaming: every tile through the general instantiation (no plain-tile kernel beside it)
@@ -154,7 +156,7 @@ struct KernelConfig {
 constexpr int kTuneCandidates[][5] = {{1, 8, 6, 0, 0}, {1, 8, 8, 0, 0},  {1, 8, 4, 0, 0}, {1, 8, 6, 32, 0},
                                       {1, 12, 4, 0, 0}, {1, 6, 6, 0, 0}, {1, 4, 6, 0, 0}, {1, 4, 6, 16, 0},
                                       {1, 8, 6, 4, 0}, {1, 4, 6, 4, 0},  {1, 8, 6, 0, 1}, {1, 8, 6, 4, 1},
-                                      {1, 4, 6, 4, 1}};
+                                      {1, 4, 6, 4, 1}, {3, 128, 0, 0, 0}, {3, 256, 0, 0, 0}};
 using TuneChoice = std::array<int, 5>;
 std::mutex g_tune_mutex;
 std::map<std::vector<int>, TuneChoice> g_tune_cache;
@@ -169,7 +171,7 @@ int one_list_env() {
 KernelConfig default_config() {
   KernelConfig c;
   if (const char* v = std::getenv("RFN_FDTD_KERNEL"))
-    c.variant = std::string(v) == "plain" ? 0 : 1;
+    c.variant = std::string(v) == "plain" ? 0 : std::string(v) == "half" ? 3 : 1;
   if (const char* v = std::getenv("RFN_FDTD_TY")) c.ty = std::atoi(v);
   if (const char* v = std::getenv("RFN_FDTD_STAGES")) c.stages = std::atoi(v);
   if (const char* v = std::getenv("RFN_FDTD_ZCHUNK")) c.zchunk = std::atoi(v);
@@ -465,6 +467,23 @@ struct ResidentClass {
   }
 };
 
+// Launch shape of the half-step kernels.
+struct HalfClass {
+  int threads = 0, seg = 0, rows = 0;
+  dim3 grid;
+  DevBuf<SimDev> d_sims;    // several simulations
+  DevBuf<int4> d_blocks;
+  DevBuf<CapSim> d_caps;    // per simulation, while a launch records histories
+  DevBuf<int> d_boxes;      // per simulation, of segment replays
+  void reset() {
+    threads = 0;
+    d_sims.free();
+    d_blocks.free();
+    d_caps.free();
+    d_boxes.free();
+  }
+};
+
 constexpr uint32_t kResSmemMax = 232448 - 4096;  // dynamic shared bytes beside the kernel's static arrays
 
 struct Engine {
@@ -473,6 +492,7 @@ struct Engine {
   KernelConfig cfg;        // the kernel in use
   StreamClass scls;        // streaming kernel
   ResidentClass res;       // resident kernel
+  HalfClass half;          // half-step kernels
   DevBuf<SimDev> d_sims;   // plain kernel
   DevBuf<int4> d_tiles;    // plain kernel
   DevBuf<int> d_err;
@@ -611,12 +631,16 @@ struct Engine {
     return tiles;
   }
 
-  // Tiles of the streaming kernel, or bricks of the resident one.
+  // Tiles of the streaming kernel, bricks of the resident one or blocks of the
+  // half-step kernels.
   void build_shape(int n_sm) {
     res.reset();
     scls.reset();
+    half.reset();
     if (cfg.variant == 2)
       build_resident(n_sm);
+    else if (cfg.variant == 3)
+      build_half();
     else
       build_stream_tiles(n_sm);
   }
@@ -777,8 +801,129 @@ struct Engine {
                                    res.smem, st));
   }
 
+  // Threads per row piece and rows per block of half-step blocks of at most t
+  // threads over rows of nx cells.
+  static void half_shape(int nx, int ny, int t, int* seg, int* rows) {
+    if (nx > t) {
+      const int pieces = (nx + t - 1) / t;
+      *seg = std::min(t, ((nx + pieces - 1) / pieces + 31) / 32 * 32);
+      *rows = 1;
+    } else {
+      *seg = nx;
+      *rows = std::min(std::max(1, t / nx), ny);
+    }
+  }
+
+  void build_half() {
+    HalfClass& c = half;
+    const int want = std::min(std::max(cfg.ty, 64), kHalfThreads) / 32 * 32;
+    if (sims.size() == 1) {
+      const fdtd_sim* s = sims[0];
+      half_shape(s->nx, s->ny, want, &c.seg, &c.rows);
+      c.threads = (c.seg * c.rows + 31) / 32 * 32;
+      c.grid = dim3(unsigned((s->nx + c.seg - 1) / c.seg), unsigned((s->ny + c.rows - 1) / c.rows), unsigned(s->nz));
+      n_tiles = grid = int(std::min<int64_t>(int64_t(c.grid.x) * c.grid.y * c.grid.z, INT_MAX));
+    } else {
+      // the block size that leaves the fewest threads idle over all grids
+      double best = -1.0;
+      for (int t = std::max(64, want / 2); t <= kHalfThreads; t += 32) {
+        double used = 0, all = 0;
+        for (auto* s : sims) {
+          int seg, rows;
+          half_shape(s->nx, s->ny, t, &seg, &rows);
+          used += double(s->nx) * s->ny * s->nz;
+          all += double((s->nx + seg - 1) / seg) * ((s->ny + rows - 1) / rows) * s->nz * t;
+        }
+        if (used / all > best) {
+          best = used / all;
+          c.threads = t;
+        }
+      }
+      std::vector<int4> blocks;
+      std::vector<SimDev> devs;
+      for (size_t i = 0; i < sims.size(); ++i) {
+        const fdtd_sim* s = sims[i];
+        devs.push_back(s->dev);
+        int seg, rows;
+        half_shape(s->nx, s->ny, c.threads, &seg, &rows);
+        for (int z = 0; z < s->nz; ++z)
+          for (int y0 = 0; y0 < s->ny; y0 += rows)
+            for (int x0 = 0; x0 < s->nx; x0 += seg)
+              blocks.push_back(make_int4(int(i), x0 | (rows << 16), y0, z | (seg << 16)));
+      }
+      if (blocks.size() > size_t(INT_MAX)) throw ArgError{FDTD_ERR_LIMIT, "Too many half-step blocks."};
+      c.grid = dim3(unsigned(blocks.size()));
+      c.d_sims.alloc(devs.size());
+      CK(cudaMemcpy(c.d_sims.p, devs.data(), devs.size() * sizeof(SimDev), cudaMemcpyHostToDevice));
+      c.d_blocks.alloc(blocks.size());
+      CK(cudaMemcpy(c.d_blocks.p, blocks.data(), blocks.size() * sizeof(int4), cudaMemcpyHostToDevice));
+      n_tiles = grid = int(blocks.size());
+    }
+    zchunk_used = 1;
+  }
+
+  // Per simulation of the engine: what the E launches record (all-zero: nothing).
+  void half_captures(const std::vector<CapSim>& caps) {
+    if (caps.empty()) return;
+    half.d_caps.reserve(caps.size());
+    CK(cudaMemcpy(half.d_caps.p, caps.data(), caps.size() * sizeof(CapSim), cudaMemcpyHostToDevice));
+  }
+
+  template <typename... A>
+  static void launch_dependent(void (*fn)(A...), dim3 grid, int threads, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid;
+    lc.blockDim = dim3(unsigned(threads));
+    lc.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&lc, fn, args...));
+  }
+
+  // One half of step n (E, or H) on st. cap: the E launch writes the box
+  // histories of half.d_caps at slot n - n0. reach >= 0: only the cells that
+  // half.d_boxes' boxes need when `reach` more cells around them have to be right.
+  void launch_half(cudaStream_t st, int n, bool h_side, bool cap, int n0 = 0, int reach = -1) {
+    HalfClass& c = half;
+    const bool one = sims.size() == 1;
+    HalfLaunch L{};
+    L.n = n;
+    dim3 grid = c.grid;
+    int threads = c.threads;
+    L.lo = reach + (h_side ? 0 : 1);  // H needs E of the -1 neighbours
+    L.hi = reach;
+    int w[3] = {1, 1, 1};  // the largest region along each axis
+    for (size_t i = 0; i < sims.size() && reach >= 0; ++i) {
+      const int* b = &rep_boxes[6 * i];
+      const int nn[3] = {sims[i]->nx, sims[i]->ny, sims[i]->nz};
+      for (int a = 0; a < 3; ++a)
+        w[a] = std::max(w[a], std::min(nn[a], b[2 * a + 1] + L.hi) - std::max(0, b[2 * a] - L.lo));
+    }
+    if (reach >= 0 && int64_t(w[2]) * int64_t(sims.size()) <= 65535) {
+      L.boxes = c.d_boxes.p;
+      half_shape(w[0], w[1], std::max(64, cfg.ty), &L.seg, &L.rows);
+      L.planes = w[2];
+      threads = (L.seg * L.rows + 31) / 32 * 32;
+      grid = dim3(unsigned((w[0] + L.seg - 1) / L.seg), unsigned((w[1] + L.rows - 1) / L.rows),
+                  unsigned(w[2]) * unsigned(sims.size()));
+    } else {
+      L.blocks = one ? nullptr : c.d_blocks.p;
+      L.seg = c.seg;
+      L.rows = c.rows;
+    }
+    const SimDev* ds = c.d_sims.p;
+    const CapSim* dc = c.d_caps.p;
+    auto fn = h_side ? (one ? &half_step_kernel<true, true, false> : &half_step_kernel<true, false, false>)
+              : cap  ? (one ? &half_step_kernel<false, true, true> : &half_step_kernel<false, false, true>)
+                     : (one ? &half_step_kernel<false, true, false> : &half_step_kernel<false, false, false>);
+    launch_dependent(fn, grid, threads, st, sims[0]->dev, L, ds, dc, n0);
+  }
+
   // Time buffer that holds the state before step n.
-  int state_buf(int n) const { return cfg.variant == 2 ? 0 : n & 1; }
+  int state_buf(int n) const { return cfg.variant >= 2 ? 0 : n & 1; }
 
   // Picks the step kernel and its shape for this set of grids: each candidate
   // runs a few time steps on the simulations themselves (their fields are
@@ -1078,6 +1223,10 @@ struct Engine {
     } else if (cfg.variant == 2) {
       launch_resident(st, n, n + 1);
       return 1;
+    } else if (cfg.variant == 3) {
+      launch_half(st, n, false, false);
+      launch_half(st, n, true, false);
+      return 1;
     } else {
       fdtd_step_kernel<kTileY><<<n_tiles, dim3(32, kBlockY), 0, st>>>(d_sims.p, d_tiles.p, n);
       CK(cudaGetLastError());
@@ -1173,6 +1322,12 @@ struct Engine {
         nb_max = std::max(nb_max, c.nb);
         v.push_back(c);
       }
+    if (cfg.variant == 3 && !v.empty()) {
+      std::vector<CapSim> hc(sims.size(), CapSim{});
+      for (size_t i = 0, k = 0; i < sims.size(); ++i)
+        if (sims[i]->adj_mode == 2) hc[i] = v[k++];
+      half_captures(hc);
+    }
     n_caps = int(v.size());
     d_caps.alloc(v.size());
     if (!v.empty()) CK(cudaMemcpy(d_caps.p, v.data(), v.size() * sizeof(CapSim), cudaMemcpyHostToDevice));
@@ -1191,6 +1346,7 @@ struct Engine {
   // gradient box, nearest first, with those distances (cells).
   DevBuf<StreamTile> rep_tiles, rep_tiles_p;
   std::vector<int> rep_dist, rep_dist_p;
+  std::vector<int> rep_boxes;      // gradient box of each simulation of the engine (empty: none)
   std::vector<std::unique_ptr<AdjBufs>> adj_bufs;
   DevBuf<AdjSim> adj_d_as;
   DevBuf<int4> adj_d_t;
@@ -1455,7 +1611,21 @@ struct Engine {
       // box: with the streaming kernels each replay step runs the tiles within
       // that reach (nearest first). Tiles outside it keep stale values, which
       // never reach what the history reads before the segment ends.
-      const bool cone = cfg.variant == 1 && !std::getenv("RFN_REPLAY_FULL");
+      const bool full = std::getenv("RFN_REPLAY_FULL") != nullptr;
+      const bool cone = cfg.variant == 1 && !full, half_cone = cfg.variant == 3 && !full;
+      if (cfg.variant == 3) {
+        std::vector<CapSim> hc(sims.size(), CapSim{});
+        rep_boxes.assign(6 * sims.size(), 0);
+        for (size_t q = 0; q < req.size(); ++q)
+          for (size_t i = 0; i < sims.size(); ++i)
+            if (sims[i] == req[q].s) {
+              hc[i] = caps[q];
+              std::copy(req[q].box, req[q].box + 6, rep_boxes.begin() + 6 * std::ptrdiff_t(i));
+            }
+        half_captures(hc);
+        half.d_boxes.reserve(rep_boxes.size());
+        CK(cudaMemcpy(half.d_boxes.p, rep_boxes.data(), rep_boxes.size() * sizeof(int), cudaMemcpyHostToDevice));
+      }
       if (cone) {
         std::vector<const int*> boxes(sims.size(), nullptr);
         for (const auto& r : req)
@@ -1474,7 +1644,7 @@ struct Engine {
       // each step's box capture beside it (as in a recorded run)
       auto replay = [&](int k) {
         const int n0 = k * K, n1 = std::min(nt, n0 + K), h0 = n0 - (k & 1) * K;
-        const size_t b = size_t(n0 & 1);
+        const size_t b = size_t(state_buf(n0));
         for (const auto& r : req) {
           fdtd_sim* s = r.s;
           const size_t N = s->cells_padded;
@@ -1488,6 +1658,13 @@ struct Engine {
         if (cfg.variant == 1) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), rs));
         unsigned base_g = 0, base_p = 0;
         for (int n = n0; n < n1; ++n) {
+          if (cfg.variant == 3) {
+            // E of the segment's last step is advanced only for its history
+            const int reach = half_cone ? n1 - 1 - n : -1;
+            launch_half(rs, n, false, true, h0, reach);
+            if (n + 1 < n1) launch_half(rs, n, true, false, 0, reach);
+            continue;
+          }
           CK(cudaEventRecord(cap_fork, rs));
           CK(cudaStreamWaitEvent(cap_stream, cap_fork, 0));
           adj_capture_kernel<<<dim3(cap_grid, unsigned(caps.size())), 256, 0, cap_stream>>>(d_c.p, n, h0);
@@ -1528,9 +1705,20 @@ struct Engine {
     CK(cudaEventElapsedTime(&ms, ev0, ev1));
     adj_ms = ms;
     check_error();
-    for (size_t i = 0; i < req.size(); ++i)
-      CK(cudaMemcpy(req[i].grad_out, adj_bufs[i]->grad.p, adj_bufs[i]->grad.n * sizeof(double),
-                    cudaMemcpyDeviceToHost));
+    // the device's box arrays run x fastest, the caller's z fastest
+    std::vector<double> g;
+    for (size_t i = 0; i < req.size(); ++i) {
+      const int* b = req[i].box;
+      const int bx = b[1] - b[0], by = b[3] - b[2], bz = b[5] - b[4];
+      g.resize(adj_bufs[i]->grad.n);
+      CK(cudaMemcpy(g.data(), adj_bufs[i]->grad.p, g.size() * sizeof(double), cudaMemcpyDeviceToHost));
+      double* out = req[i].grad_out;
+      for (int k = 0; k < 9; ++k, out += box_cells(b))
+        for (int x = 0; x < bx; ++x)
+          for (int y = 0; y < by; ++y)
+            for (int z = 0; z < bz; ++z)
+              out[(size_t(x) * by + y) * bz + z] = g[size_t(k) * size_t(box_cells(b)) + size_t(box_cell(x, y, z, bx, by))];
+    }
   }
 
   // Enqueue one full run of nt steps on stream st (used for capture and for
@@ -1575,7 +1763,7 @@ struct Engine {
     for (int n = 0; n < nt && cfg.variant != 2; ++n) {
       for (auto* s : sims)
         if (s->ckpt_every > 0 && n % s->ckpt_every == 0 && s->ckpt.n) {
-          const size_t N = s->cells_padded, b = size_t(n & 1);
+          const size_t N = s->cells_padded, b = size_t(state_buf(n));
           const size_t sb = s->splits.n ? 2 * s->split_buf_pairs : 0;  // split floats per time buffer
           const size_t stride = 6 * N + sb;
           float* dst = s->ckpt.p + size_t(n / s->ckpt_every) * stride;
@@ -1583,7 +1771,11 @@ struct Engine {
           if (sb)
             CK(cudaMemcpyAsync(dst + 6 * N, s->splits.p + b * sb, sb * sizeof(float), cudaMemcpyDeviceToDevice, st));
         }
-      if (n_caps) {
+      if (cfg.variant == 3) {  // the E launch writes the box history of its step
+        launch_half(st, n, false, n_caps > 0);
+        launch_half(st, n, true, false);
+        ++step_launches;
+      } else if (n_caps) {
         // the box history of step n reads buffer n & 1, which step n only
         // reads and step n+1 overwrites: it runs on a side stream beside step n
         CK(cudaEventRecord(cap_fork, st));
@@ -1592,11 +1784,12 @@ struct Engine {
         CK(cudaGetLastError());
         CK(cudaEventRecord(cap_join, cap_stream));
       }
-      step_launches += launch_step(st, n);
-      if (n_caps) CK(cudaStreamWaitEvent(st, cap_join, 0));
+      if (cfg.variant != 3) step_launches += launch_step(st, n);
+      if (n_caps && cfg.variant != 3) CK(cudaStreamWaitEvent(st, cap_join, 0));
       // The monitors of step n read the buffer that step n + 1 only reads: they
       // run on a side stream beside it, and step n + 2, which overwrites that
-      // buffer, waits for them.
+      // buffer, waits for them. (The half steps work in place: there the next
+      // step waits.)
       if (mon_pending) {
         CK(cudaStreamWaitEvent(st, mon_join, 0));
         mon_pending = false;
@@ -1612,11 +1805,12 @@ struct Engine {
             int most = 1;
             for (const auto& m : s->monitors) most = std::max(most, m.n1 * m.n2);
             monitor_kernel<<<dim3(unsigned(std::min(64, (most + 127) / 128)), unsigned(s->monitors.size())), 128, 0,
-                             mon_stream>>>(s->d_dev.p, s->d_mons.p, n, (n + 1) & 1);
+                             mon_stream>>>(s->d_dev.p, s->d_mons.p, n, state_buf(n + 1));
             CK(cudaGetLastError());
           }
         CK(cudaEventRecord(mon_join, mon_stream));
-        mon_pending = true;
+        mon_pending = cfg.variant != 3;
+        if (!mon_pending) CK(cudaStreamWaitEvent(st, mon_join, 0));
       }
       if ((n + 1) % kDftChunk == 0 || n + 1 == nt) dft_upto(n + 1);
     }
