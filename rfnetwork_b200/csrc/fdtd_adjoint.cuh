@@ -348,15 +348,18 @@ adj_step_kernel(const AdjSim* __restrict__ sims, const int4* __restrict__ tiles,
 }
 
 // Adjoints of the records of step `step` into buffer `buf` (the start of the
-// reverse sweep; later steps add theirs inside adj_step_kernel). One block
-// row per simulation.
-__global__ void adj_inject_kernel(const AdjSim* __restrict__ sims, int step, int buf) {
+// reverse sweep; later steps add theirs inside the reverse step) of the fields
+// from field0 on (3: H only, for the half-step reverse, which adds the E records
+// itself).
+// One block row per simulation.
+__global__ void adj_inject_kernel(const AdjSim* __restrict__ sims, int step, int buf, int field0) {
   const AdjSim& A = sims[blockIdx.y];
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= A.n_probes) return;
   const float rv = A.radj[size_t(p) * A.nt + step];
   if (rv == 0.f) return;
   const int idx = A.probe_idx[p], f = A.probe_field[p];
+  if (f < field0) return;
   const uint32_t fl = adj_flags(A.rows + 8 * A.mat[idx]);
   const int64_t N = A.N;
   // field f: total f of [E totals, H totals], or halves 2f, 2f+1 of the 12 halves

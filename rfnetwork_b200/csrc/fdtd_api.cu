@@ -30,6 +30,7 @@
 #include "fdtd_nf2ff.cuh"
 #include "fdtd_step_stream.cuh"
 #include "fdtd_half.cuh"
+#include "fdtd_adjoint_half.cuh"
 #include "fdtd_resident.cuh"
 #include "fdtd_adjoint_stream.cuh"
 #include <cudaTypedefs.h>
@@ -814,6 +815,37 @@ struct Engine {
     }
   }
 
+  // Blocks over every cell of every simulation, of the size around `want`
+  // threads that leaves the fewest idle over all grids; returns that size.
+  int half_blocks(int want, std::vector<int4>& blocks) const {
+    double best = -1.0;
+    int threads = want;
+    for (int t = std::max(64, want / 2); t <= kHalfThreads; t += 32) {
+      double used = 0, all = 0;
+      for (auto* s : sims) {
+        int seg, rows;
+        half_shape(s->nx, s->ny, t, &seg, &rows);
+        used += double(s->nx) * s->ny * s->nz;
+        all += double((s->nx + seg - 1) / seg) * ((s->ny + rows - 1) / rows) * s->nz * t;
+      }
+      if (used / all > best) {
+        best = used / all;
+        threads = t;
+      }
+    }
+    for (size_t i = 0; i < sims.size(); ++i) {
+      const fdtd_sim* s = sims[i];
+      int seg, rows;
+      half_shape(s->nx, s->ny, threads, &seg, &rows);
+      for (int z = 0; z < s->nz; ++z)
+        for (int y0 = 0; y0 < s->ny; y0 += rows)
+          for (int x0 = 0; x0 < s->nx; x0 += seg)
+            blocks.push_back(make_int4(int(i), x0 | (rows << 16), y0, z | (seg << 16)));
+    }
+    if (blocks.size() > size_t(INT_MAX)) throw ArgError{FDTD_ERR_LIMIT, "Too many half-step blocks."};
+    return threads;
+  }
+
   void build_half() {
     HalfClass& c = half;
     const int want = std::min(std::max(cfg.ty, 64), kHalfThreads) / 32 * 32;
@@ -824,34 +856,10 @@ struct Engine {
       c.grid = dim3(unsigned((s->nx + c.seg - 1) / c.seg), unsigned((s->ny + c.rows - 1) / c.rows), unsigned(s->nz));
       n_tiles = grid = int(std::min<int64_t>(int64_t(c.grid.x) * c.grid.y * c.grid.z, INT_MAX));
     } else {
-      // the block size that leaves the fewest threads idle over all grids
-      double best = -1.0;
-      for (int t = std::max(64, want / 2); t <= kHalfThreads; t += 32) {
-        double used = 0, all = 0;
-        for (auto* s : sims) {
-          int seg, rows;
-          half_shape(s->nx, s->ny, t, &seg, &rows);
-          used += double(s->nx) * s->ny * s->nz;
-          all += double((s->nx + seg - 1) / seg) * ((s->ny + rows - 1) / rows) * s->nz * t;
-        }
-        if (used / all > best) {
-          best = used / all;
-          c.threads = t;
-        }
-      }
       std::vector<int4> blocks;
       std::vector<SimDev> devs;
-      for (size_t i = 0; i < sims.size(); ++i) {
-        const fdtd_sim* s = sims[i];
-        devs.push_back(s->dev);
-        int seg, rows;
-        half_shape(s->nx, s->ny, c.threads, &seg, &rows);
-        for (int z = 0; z < s->nz; ++z)
-          for (int y0 = 0; y0 < s->ny; y0 += rows)
-            for (int x0 = 0; x0 < s->nx; x0 += seg)
-              blocks.push_back(make_int4(int(i), x0 | (rows << 16), y0, z | (seg << 16)));
-      }
-      if (blocks.size() > size_t(INT_MAX)) throw ArgError{FDTD_ERR_LIMIT, "Too many half-step blocks."};
+      for (auto* s : sims) devs.push_back(s->dev);
+      c.threads = half_blocks(want, blocks);
       c.grid = dim3(unsigned(blocks.size()));
       c.d_sims.alloc(devs.size());
       CK(cudaMemcpy(c.d_sims.p, devs.data(), devs.size() * sizeof(SimDev), cudaMemcpyHostToDevice));
@@ -1354,6 +1362,9 @@ struct Engine {
   DevBuf<AdjMaps> adj_d_maps;     // streaming reverse step: tensor maps of each simulation's adjoint state
   DevBuf<int4> adj_d_ts;          // its tiles (w: the tile's boxes hold split cells)
   DevBuf<unsigned> adj_counter;   // its tile counter
+  DevBuf<int4> adj_d_blocks;      // half-step reverse: blocks over several simulations
+  static constexpr int kAdjHalfWant = 128;                // its threads per block (64 and 256: up to 10 % slower)
+  static constexpr int64_t kAdjHalfBytes = 120'000'000;
   static int adj_tiles_per_sm() {
     const char* v = std::getenv("RFN_ADJ_TILES_PER_SM");
     return v ? std::max(1, std::atoi(v)) : 4;
@@ -1432,6 +1443,21 @@ struct Engine {
     int dev = 0, n_sm = 148;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+    const char* sv = std::getenv("RFN_ADJ_STREAM");
+    const bool stream_adj = sv && std::atoi(sv) != 0;
+    // The half-step reverse where its state (six totals per cell, six halves more
+    // per cell with split E or H) fits in L2, which then serves it twice per step;
+    // beyond that one launch per step, which reads it once. Per step, one launch
+    // against two halves: 52x44x33 cells with 6-cell layers 20.5 against 12.7 us,
+    // 96x96x64 with 10 39.6 against 31.1, 128x128x96 with 10 (74 MB) 88.9 against
+    // 71.3, 160x150x120 with 6 (98 MB) 148.6 against 139.3; 224x200x128 with 8
+    // (195 MB) 247 against 259, and a design step of six 96x96x64 members (185 MB)
+    // 105 against 111 ms. RFN_ADJ_HALF=0 / 1 decides.
+    int64_t adj_state = 0;
+    for (const auto& rq : req)
+      adj_state += 24 * (int64_t(rq.s->nx) * rq.s->ny * rq.s->nz + rq.s->grid.e_split_cells + rq.s->grid.h_split_cells);
+    const char* hv = std::getenv("RFN_ADJ_HALF");
+    const bool half_adj = !stream_adj && (hv ? std::atoi(hv) != 0 : adj_state <= kAdjHalfBytes);
     // work buffers are kept on the engine between sweeps (allocation and
     // release of ~36 floats per cell would otherwise come with every gradient)
     if (adj_bufs.size() < req.size()) adj_bufs.resize(req.size());
@@ -1457,11 +1483,12 @@ struct Engine {
         pidx[size_t(pr)] = z * s->ny * s->pitch + y * s->pitch + x;
         pfld[size_t(pr)] = s->probes[size_t(pr)].field;
       }
-      B->lam.reserve(12 * N);
-      CK(cudaMemsetAsync(B->lam.p, 0, 12 * N * sizeof(float), st));
+      // (the half-step reverse works in place, in the first of the two buffers)
+      B->lam.reserve((half_adj ? 6 : 12) * N);
+      CK(cudaMemsetAsync(B->lam.p, 0, B->lam.n * sizeof(float), st));
       if (s->splits.n) {
-        B->lams.reserve(24 * N);
-        CK(cudaMemsetAsync(B->lams.p, 0, 24 * N * sizeof(float), st));
+        B->lams.reserve((half_adj ? 12 : 24) * N);
+        CK(cudaMemsetAsync(B->lams.p, 0, B->lams.n * sizeof(float), st));
       }
       B->radj.reserve(radj.size());
       CK(cudaMemcpy(B->radj.p, radj.data(), radj.size() * sizeof(float), cudaMemcpyHostToDevice));
@@ -1513,8 +1540,6 @@ struct Engine {
     // simulation's adjoint state and material index, plane slots sized for
     // two blocks per SM.
     using AG = AdjGeom<kAdjStreamTileY>;
-    const char* sv = std::getenv("RFN_ADJ_STREAM");
-    const bool stream_adj = sv && std::atoi(sv) != 0;
     int n_ts = 0, adj_grid = 0, adj_slots = 0;
     uint32_t adj_smem = 0;
     unsigned adj_base = 0;
@@ -1562,8 +1587,35 @@ struct Engine {
       adj_counter.reserve(1);
       CK(cudaMemsetAsync(adj_counter.p, 0, sizeof(unsigned), st));
     }
+    // The half-step reverse: blocks of about 128 threads over every simulation.
+    HalfLaunch hl{};
+    dim3 half_grid;
+    int half_threads = 0;
+    if (half_adj) {
+      if (as.size() == 1) {
+        half_shape(as[0].nx, as[0].ny, kAdjHalfWant, &hl.seg, &hl.rows);
+        half_threads = (hl.seg * hl.rows + 31) / 32 * 32;
+        half_grid = dim3(unsigned((as[0].nx + hl.seg - 1) / hl.seg), unsigned((as[0].ny + hl.rows - 1) / hl.rows),
+                         unsigned(as[0].nz));
+      } else {
+        std::vector<int4> blocks;
+        half_threads = half_blocks(kAdjHalfWant, blocks);
+        half_grid = dim3(unsigned(blocks.size()));
+        adj_d_blocks.reserve(blocks.size());
+        CK(cudaMemcpy(adj_d_blocks.p, blocks.data(), blocks.size() * sizeof(int4), cudaMemcpyHostToDevice));
+        hl.blocks = adj_d_blocks.p;
+      }
+    }
     auto reverse_step = [&](int n, int hist_n0) {
-      if (stream_adj) {
+      if (half_adj) {
+        const bool one = as.size() == 1;
+        hl.n = n;
+        const AdjSim* ds = adj_d_as.p;
+        launch_dependent(one ? &adj_half_kernel<false, true> : &adj_half_kernel<false, false>, half_grid, half_threads,
+                         st, as[0], hl, ds, hist_n0);
+        launch_dependent(one ? &adj_half_kernel<true, true> : &adj_half_kernel<true, false>, half_grid, half_threads,
+                         st, as[0], hl, ds, hist_n0);
+      } else if (stream_adj) {
         adj_stream_kernel<kAdjStreamTileY><<<adj_grid, AG::THREADS, adj_smem, st>>>(
             adj_d_as.p, adj_d_maps.p, adj_d_ts.p, n_ts, n, hist_n0, adj_counter.p, adj_base, d_err.p, adj_slots,
             wait_limit);
@@ -1590,8 +1642,8 @@ struct Engine {
     }
     const int cap_grid = int(std::min<int64_t>(1024, std::max<int64_t>(1, (nb_max + 255) / 256)));
     if (p_max > 0) {
-      adj_inject_kernel<<<dim3((p_max + 127) / 128, unsigned(as.size())), 128, 0, st>>>(d_as.p, nt - 1,
-                                                                                        (nt - 1) & 1);
+      adj_inject_kernel<<<dim3((p_max + 127) / 128, unsigned(as.size())), 128, 0, st>>>(
+          d_as.p, nt - 1, half_adj ? 0 : (nt - 1) & 1, half_adj ? 3 : 0);
       CK(cudaGetLastError());
     }
     adj_launches = 0;

@@ -86,14 +86,18 @@ def test_batch_equals_single_runs(engine_lib, monkeypatch):
 
 @pytest.mark.parametrize("mode", ["recorded", "checkpointed", "checkpointed, whole grid"])
 def test_gradients_equal_plain(engine_lib, monkeypatch, mode):
-    """Histories written by the E launches, and segment replays of the cells
-    within reach of the box, against a plain-kernel run of the same mode."""
+    """Histories written by the E launches, segment replays of the cells within
+    reach of the box and the half-step reverse, against a plain-kernel run of the
+    same mode and the reverse step in one launch."""
     s = configs.microstrip(n=(58, 44, 30), n_pml=5, nt=130)
     box = (24, 33, 18, 26, 12, 15)
     if mode.endswith("grid"):
         monkeypatch.setenv("RFN_REPLAY_FULL", "1")
 
+    halves = iter(("1", "0"))
+
     def run(sim):
+        monkeypatch.setenv("RFN_ADJ_HALF", next(halves))
         if mode == "recorded":
             sim.run_recorded(130, box)
         else:
@@ -114,6 +118,7 @@ def test_batched_gradients_equal_single(engine_lib, monkeypatch):
     out = {}
     for kernel in ("half", "plain"):
         monkeypatch.setenv("RFN_FDTD_KERNEL", kernel)
+        monkeypatch.setenv("RFN_ADJ_HALF", "1" if kernel == "half" else "0")
         sims = [_model_sim(s)[0] for s in models]
         b = _lib.Batch(sims)
         for mode in ("recorded", "checkpointed"):
