@@ -289,6 +289,12 @@ void d2h(fdtd_sim* s, void* dst, const void* src, size_t bytes) {
   s->d2h_bytes += int64_t(bytes);
 }
 
+// Waits for the uploads issued so far. A copy from pageable memory returns when
+// the host buffer may be reused, before its last bytes are on the device, and
+// the engine's streams don't wait for the legacy stream by themselves: this
+// comes between the uploads and the first kernel on another stream.
+void uploads_done() { CK(cudaStreamSynchronize(0)); }
+
 using StreamKernelFn = void (*)(const SimDev*, const StreamTile*, int, int, unsigned*, unsigned, int*, int, int,
                                 uint32_t, int);
 
@@ -1004,6 +1010,7 @@ struct Engine {
     float best_ms = 1e30f;
     for (const auto& c : cand) {
       if (!build(c)) continue;
+      uploads_done();
       if (scls.d_counter.n) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), st));
       launch_steps(st, 0, warm);
       CK(cudaEventRecord(ev0, st));
@@ -1641,6 +1648,7 @@ struct Engine {
       CK(cudaMemcpy(d_c.p, caps.data(), caps.size() * sizeof(CapSim), cudaMemcpyHostToDevice));
     }
     const int cap_grid = int(std::min<int64_t>(1024, std::max<int64_t>(1, (nb_max + 255) / 256)));
+    uploads_done();
     if (p_max > 0) {
       adj_inject_kernel<<<dim3((p_max + 127) / 128, unsigned(as.size())), 128, 0, st>>>(
           d_as.p, nt - 1, half_adj ? 0 : (nt - 1) & 1, half_adj ? 3 : 0);
@@ -1685,6 +1693,7 @@ struct Engine {
             if (sims[i] == r.s) boxes[i] = r.box;
         build_replay_tiles(boxes);
       }
+      uploads_done();
       // the replays rewrite probe records (outside the reach, with stale
       // values): the forward's records are kept aside and put back at the end
       for (size_t i = 0; i < req.size(); ++i) {
@@ -1887,6 +1896,7 @@ struct Engine {
     if (!use_graph) {  // every launch issued from the host, step by step
       reset_graph();
       build_caps();
+      uploads_done();
       CK(cudaEventRecord(ev0, st));
       enqueue(st, nt);
       CK(cudaEventRecord(ev1, st));
@@ -1916,6 +1926,7 @@ struct Engine {
       cudaStreamDestroy(cap);
       graph_nt = nt;
     }
+    uploads_done();
     CK(cudaEventRecord(ev0, st));
     CK(cudaGraphLaunch(graph, st));
     CK(cudaEventRecord(ev1, st));
