@@ -232,9 +232,12 @@ int fdtd_adjoint(fdtd_sim* s, const double* dJ_dX, int n_series, int n_freq, con
 
 /* ---------------------------------------------------------------- batches */
 
-/* Many independent simulations of uneven sizes stepped together: one kernel
- * launch per time step covers the tile work lists of all members, and the time
- * loop is captured as a CUDA graph. The reference has no batched engine; its
+/* Many independent simulations of uneven sizes run by one call. Small members
+ * step together, one launch covering the work lists of them all; members that
+ * fill the GPU alone run one after the other (a kernel chosen with
+ * fdtd_batch_set_kernel steps all members together). The time loops are captured
+ * as CUDA graphs. The statistics count a step of all members as one launch.
+ * The reference has no batched engine; its
  * counterpart is one solver_run_cu call per simulation
  * (rfnetwork/core/src/cuda_binding.cpp:20-68). Members keep their own
  * coefficients, probes and DFT; results are read per member after the run. */
@@ -248,9 +251,9 @@ int fdtd_batch_get_stats(const fdtd_batch* b, fdtd_stats* out);
  * fdtd_run_recorded for every member, boxes = n_sims x 6 ints;
  * fdtd_batch_run_checkpointed is fdtd_run_checkpointed for every member (state
  * snapshots every `every` steps), with the boxes fixed at the run. Then
- * fdtd_batch_adjoint runs the adjoints of all members together, one launch per
- * reverse step over all their tiles; after a checkpointed run it replays each
- * segment of all members with one step launch per time step. dJ_dX[i] and
+ * fdtd_batch_adjoint runs the adjoints of the members that step together in the
+ * same launches, after a checkpointed run with the replays of their segments
+ * beside them. dJ_dX[i] and
  * grad[i] are member i's arrays, sized as for fdtd_adjoint by its own DFT and
  * box. */
 int fdtd_batch_run_recorded(fdtd_batch* b, int nt, const int* boxes);

@@ -336,7 +336,7 @@ class Simulation:
 
 
 class Batch:
-    """Several simulations stepped together by one kernel launch per step."""
+    """Several simulations run by one call: small ones share launches, large ones run one after the other."""
 
     def __init__(self, sims):
         self.lib = load()

@@ -491,6 +491,9 @@ struct HalfClass {
   }
 };
 
+// cells below which a batch's members step together, and the most cells of such a part
+constexpr int64_t kBatchSmallRun = 40'000, kBatchSmallGradient = 256'000, kBatchCells = 1'200'000;
+
 constexpr uint32_t kResSmemMax = 232448 - 4096;  // dynamic shared bytes beside the kernel's static arrays
 
 struct Engine {
@@ -533,7 +536,7 @@ struct Engine {
   cudaStream_t stream() const { return ext_stream ? ext_stream : own_stream; }
 
   void init() {
-    if (!own_stream) CK(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
+    if (!own_stream && !ext_stream) CK(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
     if (!ev0) CK(cudaEventCreate(&ev0));
     if (!ev1) CK(cudaEventCreate(&ev1));
     if (!cap_stream) CK(cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
@@ -2218,14 +2221,116 @@ void check_gradient_box(const fdtd_sim* s, const int* box) {
       }
 }
 
+// The members of a batch run in parts, one part after the other on one stream,
+// the members of a part in the same launches.
 struct fdtd_batch {
   std::vector<fdtd_sim*> sims;
-  Engine engine;
+  KernelConfig asked;
+  cudaStream_t ext_stream = nullptr;
+  std::vector<std::unique_ptr<Engine>> parts;
+  std::vector<std::vector<size_t>> members;  // of each part
+  int run_nt = -1;        // steps the parts' graphs were made for
   bool dirty = true;
-  std::vector<int> gens;  // members' device-buffer generations the engine was built on
+  std::vector<int> gens;  // members' device-buffer generations the parts were built on
   std::string err;
   fdtd_stats stats{};
 };
+
+// Which members step together. Members are independent, so one that fills the
+// GPU alone is best stepped alone: it takes the kernel that suits it (the
+// resident one holds up to half a million cells) and its state stays in L2,
+// while all states together do not. Eight members of 0.12 to 1.1 M cells: 151 us
+// per step together, 102 one after the other. Small members share launches,
+// whose latency is then paid once. Per member and step, together against alone,
+// 22k cells 3.7 (two members), 2.0 (four), 1.2 (32) against 3.0 us, 47k cells
+// 3.3 (four) and 2.6 (16) against 3.1 us, 85k cells 4.8 against 4.2 us. For a
+// gradient, whose steps are two or four launches: four members of 75k cells 14.9
+// against 21.8 ms, 192k cells 24.8 against 28.9 ms, 346k cells 39.9 against 35.3
+// ms; six of 590k cells 96 against 78 ms.
+std::vector<std::vector<size_t>> batch_parts(const fdtd_batch* b) {
+  std::vector<std::vector<size_t>> out;
+  std::vector<size_t> small;
+  auto cells = [&](size_t i) { return int64_t(b->sims[i]->nx) * b->sims[i]->ny * b->sims[i]->nz; };
+  const bool automatic = b->asked.variant == 1 && b->asked.ty == 0, run = b->sims[0]->adj_mode == 0;
+  for (size_t i = 0; i < b->sims.size(); ++i) {
+    if (!automatic || cells(i) < (run ? kBatchSmallRun : kBatchSmallGradient))
+      small.push_back(i);
+    else
+      out.push_back({i});
+  }
+  int64_t room = 0;
+  for (size_t i : small) {
+    const bool together = !automatic || !run || small.size() > 2;
+    if (!together || (automatic && room < cells(i)) || room == 0) {
+      out.emplace_back();
+      room = kBatchCells;
+    }
+    out.back().push_back(i);
+    room -= automatic ? cells(i) : 0;
+  }
+  return out;
+}
+
+// All parts use one stream: the caller's, or the first part's own.
+void set_batch_streams(fdtd_batch* b) {
+  for (auto& e : b->parts) {
+    e->ext_stream = e == b->parts[0] ? b->ext_stream : b->parts[0]->stream();
+    e->init();
+  }
+}
+
+// (Re)builds the parts for the members as prepared.
+void build_batch(fdtd_batch* b, int nt) {
+  auto members = batch_parts(b);
+  if (members != b->members) {
+    for (auto& e : b->parts) cudaStreamSynchronize(e->stream());
+    b->parts.clear();
+    b->members = std::move(members);
+    for (const auto& m : b->members) {
+      b->parts.push_back(std::make_unique<Engine>());
+      for (size_t i : m) b->parts.back()->sims.push_back(b->sims[i]);
+    }
+  }
+  b->run_nt = -1;
+  set_batch_streams(b);
+  for (auto& e : b->parts) {
+    e->asked = b->asked;
+    e->graph_nt = -1;
+    e->build_tiles();
+  }
+  b->run_nt = nt;
+}
+
+// Runs nt steps of every part and reports the first error after all have ended.
+void run_batch(fdtd_batch* b, int nt) {
+  std::exception_ptr first;
+  set_batch_streams(b);
+  for (auto& e : b->parts) e->run_async(nt);
+  for (auto& e : b->parts) {
+    try {
+      e->sync();
+    } catch (...) {
+      if (!first) first = std::current_exception();
+    }
+  }
+  if (first) std::rethrow_exception(first);
+  for (size_t k = 0; k < b->parts.size(); ++k)
+    for (size_t i : b->members[k]) fill_stats(b->sims[i], b->parts[k].get());
+}
+
+// Times and trials summed over the parts; a launch of every part counts once.
+void batch_run_stats(fdtd_batch* b, int nt) {
+  fdtd_stats& st = b->stats;
+  st.nt = nt;
+  st.last_run_ms = st.tune_ms = 0;
+  st.step_launches = st.tune_trials = 0;
+  for (const auto& e : b->parts) {
+    st.last_run_ms += e->last_ms;
+    st.tune_ms += e->tune_ms;
+    st.tune_trials += e->tune_trials;
+    st.step_launches = std::max<int64_t>(st.step_launches, e->step_launches);
+  }
+}
 
 // Whether a member's device buffers moved since the batch engine was built.
 bool batch_moved(const fdtd_batch* b) {
@@ -2747,8 +2852,7 @@ int fdtd_batch_create(fdtd_sim* const* sims, int n_sims, fdtd_batch** out) {
     }
     b->sims.push_back(sims[i]);
   }
-  b->engine.sims = b->sims;
-  b->engine.asked = default_config();
+  b->asked = default_config();
   *out = b;
   return FDTD_OK;
 }
@@ -2760,18 +2864,18 @@ int fdtd_batch_set_kernel(fdtd_batch* b, int variant, int tile_y, int stages, in
       throw ArgError{FDTD_ERR_ARG, "variant must be 0 (plain) or 1 (stream)"};
     if (!kernel_exists(variant, tile_y, stages))
       throw ArgError{FDTD_ERR_ARG, "No kernel instantiated for this variant / tile height / stage count."};
-    b->engine.asked.variant = variant;
-    b->engine.asked.ty = tile_y;
-    b->engine.asked.stages = stages;
-    b->engine.asked.zchunk = zchunk;
-    b->engine.asked.one_list = one_list_env();
+    b->asked.variant = variant;
+    b->asked.ty = tile_y;
+    b->asked.stages = stages;
+    b->asked.zchunk = zchunk;
+    b->asked.one_list = one_list_env();
     b->dirty = true;
   });
 }
 
 int fdtd_batch_set_stream(fdtd_batch* b, void* stream) {
   if (!b) return FDTD_ERR_ARG;
-  b->engine.ext_stream = static_cast<cudaStream_t>(stream);
+  b->ext_stream = static_cast<cudaStream_t>(stream);
   return FDTD_OK;
 }
 
@@ -2779,7 +2883,7 @@ int fdtd_batch_run(fdtd_batch* b, int nt) {
   if (!b) return FDTD_ERR_ARG;
   return guarded(&b->err, [&] {
     if (nt < 1) throw ArgError{FDTD_ERR_ARG, "nt must be positive."};
-    bool rebuild = b->engine.graph_nt != nt || b->engine.n_tiles == 0 || b->dirty;
+    bool rebuild = b->run_nt != nt || b->parts.empty() || b->dirty;
     b->dirty = false;
     for (auto* s : b->sims) {
       if (!s->prepared || s->prepared_nt != nt) rebuild = true;
@@ -2796,27 +2900,24 @@ int fdtd_batch_run(fdtd_batch* b, int nt) {
     }
     if (batch_moved(b)) rebuild = true;
     if (rebuild) {
-      b->engine.graph_nt = -1;
-      b->engine.build_tiles();
+      build_batch(b, nt);
       note_generations(b);
     }
-    b->engine.run_async(nt);
-    b->engine.sync();
-    for (auto* s : b->sims) fill_stats(s, &b->engine);
+    run_batch(b, nt);
     fdtd_stats& st = b->stats;
     st = fdtd_stats{};
-    st.nt = nt;
-    st.variant = b->engine.cfg.variant;
-    st.tile_y = b->engine.cfg.variant != 0 ? b->engine.cfg.ty : kTileY;
-    st.stages = b->engine.cfg.variant != 0 ? b->engine.cfg.stages : 0;
-    st.zchunk = b->engine.zchunk_used;
-    st.grid = b->engine.grid;
-    st.n_tiles = b->engine.n_tiles;
-    st.step_launches = b->engine.step_launches;
-    st.dft_launches = b->engine.dft_launches;
-    st.last_run_ms = b->engine.last_ms;
-    st.tune_ms = b->engine.tune_ms;
-    st.tune_trials = b->engine.tune_trials;
+    batch_run_stats(b, nt);
+    // the first part's kernel
+    const Engine& e = *b->parts[0];
+    st.variant = e.cfg.variant;
+    st.tile_y = e.cfg.variant != 0 ? e.cfg.ty : kTileY;
+    st.stages = e.cfg.variant != 0 ? e.cfg.stages : 0;
+    st.zchunk = e.zchunk_used;
+    for (const auto& p : b->parts) {
+      st.grid += p->grid;
+      st.n_tiles += p->n_tiles;
+      st.dft_launches += p->dft_launches;
+    }
     for (auto* s : b->sims) {
       st.e_split_cells += s->grid.e_split_cells;
       st.h_split_cells += s->grid.h_split_cells;
@@ -2831,7 +2932,7 @@ int fdtd_batch_run_recorded(fdtd_batch* b, int nt, const int* boxes) {
   if (!b) return FDTD_ERR_ARG;
   return guarded(&b->err, [&] {
     if (nt < 1 || !boxes) throw ArgError{FDTD_ERR_ARG, "nt must be positive and the boxes given."};
-    bool rebuild = b->engine.graph_nt != nt || b->engine.n_tiles == 0 || b->dirty;
+    bool rebuild = b->run_nt != nt || b->parts.empty() || b->dirty;
     b->dirty = false;
     for (size_t i = 0; i < b->sims.size(); ++i) {
       fdtd_sim* s = b->sims[i];
@@ -2856,18 +2957,11 @@ int fdtd_batch_run_recorded(fdtd_batch* b, int nt, const int* boxes) {
     }
     if (batch_moved(b)) rebuild = true;
     if (rebuild) {
-      b->engine.graph_nt = -1;
-      b->engine.build_tiles();
+      build_batch(b, nt);
       note_generations(b);
     }
-    b->engine.run_async(nt);
-    b->engine.sync();
-    for (auto* s : b->sims) fill_stats(s, &b->engine);
-    b->stats.nt = nt;
-    b->stats.last_run_ms = b->engine.last_ms;
-    b->stats.step_launches = b->engine.step_launches;
-    b->stats.tune_ms = b->engine.tune_ms;
-    b->stats.tune_trials = b->engine.tune_trials;
+    run_batch(b, nt);
+    batch_run_stats(b, nt);
   });
 }
 
@@ -2876,7 +2970,7 @@ int fdtd_batch_run_checkpointed(fdtd_batch* b, int nt, int every, const int* box
   return guarded(&b->err, [&] {
     if (nt < 1 || every < 1 || !boxes)
       throw ArgError{FDTD_ERR_ARG, "nt and the checkpoint interval must be positive and the boxes given."};
-    bool rebuild = b->engine.graph_nt != nt || b->engine.n_tiles == 0 || b->dirty;
+    bool rebuild = b->run_nt != nt || b->parts.empty() || b->dirty;
     b->dirty = false;
     const size_t nseg = size_t((nt + every - 1) / every);
     for (size_t i = 0; i < b->sims.size(); ++i) {
@@ -2905,18 +2999,11 @@ int fdtd_batch_run_checkpointed(fdtd_batch* b, int nt, int every, const int* box
     }
     if (batch_moved(b)) rebuild = true;
     if (rebuild) {
-      b->engine.graph_nt = -1;
-      b->engine.build_tiles();
+      build_batch(b, nt);
       note_generations(b);
     }
-    b->engine.run_async(nt);
-    b->engine.sync();
-    for (auto* s : b->sims) fill_stats(s, &b->engine);
-    b->stats.nt = nt;
-    b->stats.last_run_ms = b->engine.last_ms;
-    b->stats.step_launches = b->engine.step_launches;
-    b->stats.tune_ms = b->engine.tune_ms;
-    b->stats.tune_trials = b->engine.tune_trials;
+    run_batch(b, nt);
+    batch_run_stats(b, nt);
   });
 }
 
@@ -2928,16 +3015,24 @@ int fdtd_batch_adjoint(fdtd_batch* b, const double* const* dJ_dX, double* const*
     const int mode = b->sims.empty() ? 0 : b->sims[0]->adj_mode;
     for (size_t i = 0; i < b->sims.size(); ++i) {
       fdtd_sim* s = b->sims[i];
-      if (s->adj_mode == 0 || s->adj_mode != mode || !s->adj_in_batch || b->engine.graph_nt != s->ckpt_nt)
+      if (s->adj_mode == 0 || s->adj_mode != mode || !s->adj_in_batch || b->run_nt != s->ckpt_nt)
         throw ArgError{FDTD_ERR_STATE,
                        "fdtd_batch_adjoint needs a preceding fdtd_batch_run_recorded or fdtd_batch_run_checkpointed."};
       if (s->n_series < 1 || s->n_freq < 1) throw ArgError{FDTD_ERR_STATE, "batch member without a DFT."};
       if (!dJ_dX[i] || !grad[i]) throw ArgError{FDTD_ERR_ARG, "null member array"};
       req.push_back(Engine::AdjRequest{s, dJ_dX[i], s->adj_box, grad[i]});
     }
-    b->engine.adjoint(req);
-    b->stats.adjoint_launches = b->engine.adj_launches;
-    b->stats.adjoint_ms = b->engine.adj_ms;
+    b->stats.adjoint_launches = 0;
+    b->stats.adjoint_ms = 0;
+    set_batch_streams(b);
+    for (size_t k = 0; k < b->parts.size(); ++k) {
+      std::vector<Engine::AdjRequest> part;
+      for (size_t i : b->members[k]) part.push_back(req[i]);
+      Engine& e = *b->parts[k];
+      e.adjoint(part);
+      b->stats.adjoint_launches = std::max<int64_t>(b->stats.adjoint_launches, e.adj_launches);
+      b->stats.adjoint_ms += e.adj_ms;
+    }
   });
 }
 
@@ -2951,7 +3046,7 @@ const char* fdtd_batch_last_error(const fdtd_batch* b) { return b ? b->err.c_str
 
 void fdtd_batch_destroy(fdtd_batch* b) {
   if (!b) return;
-  cudaStreamSynchronize(b->engine.stream());
+  for (auto& e : b->parts) cudaStreamSynchronize(e->stream());
   delete b;
 }
 

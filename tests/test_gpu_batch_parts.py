@@ -1,0 +1,49 @@
+"""A batch steps its large members one after the other and its small ones
+together; each member keeps the bits of its own run either way."""
+import numpy as np
+import pytest
+
+from modelgen import configs
+from rfnetwork_b200 import _lib
+from test_gpu_resident import _model_sim
+
+pytestmark = pytest.mark.gpu
+
+NT = 60
+SMALL, MID, LARGE = (20, 18, 16), (40, 36, 34), (74, 64, 56)  # 6k, 49k and 265k cells
+BOXES = {SMALL: (8, 11, 6, 10, 5, 7), MID: (16, 24, 14, 20, 9, 11), LARGE: (30, 40, 28, 36, 12, 14)}
+
+
+@pytest.mark.parametrize("members", [
+    [SMALL], [SMALL] * 2, [SMALL] * 3, [MID, SMALL, LARGE, SMALL, SMALL], [LARGE, MID], [MID] * 3 + [LARGE] * 2])
+def test_members_keep_their_bits(engine_lib, members):
+    single = {}
+    for n in set(members):
+        m = configs.microstrip(n=n, n_pml=3, nt=NT)
+        sim, _ = _model_sim(m)
+        sim.run(NT)
+        rec = sim.probe_values()
+        sim.run_recorded(NT, BOXES[n])
+        single[n] = (m, rec, sim.adjoint(2 * sim.dft(), BOXES[n]))
+        sim.close()
+    sims = [_model_sim(single[n][0])[0] for n in members]
+    batch = _lib.Batch(sims)
+    boxes = [BOXES[n] for n in members]
+    for kind in ("run", "recorded", "checkpointed", "run"):
+        if kind == "run":
+            batch.run(NT)
+        elif kind == "recorded":
+            batch.run_recorded(NT, boxes)
+        else:
+            batch.run_checkpointed(NT, 16, boxes)
+        for n, sim in zip(members, sims):
+            assert np.abs(single[n][1]).max() > 0 and np.array_equal(sim.probe_values(), single[n][1])
+        assert batch.stats()["step_launches"] == NT
+        if kind != "run":
+            grads = batch.adjoint([2 * sim.dft() for sim in sims])
+            assert batch.stats()["adjoint_launches"] == NT
+            for n, g in zip(members, grads):
+                assert np.abs(g).max() > 0 and np.array_equal(g, single[n][2])
+    batch.close()
+    for sim in sims:
+        sim.close()
