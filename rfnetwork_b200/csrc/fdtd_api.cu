@@ -528,6 +528,7 @@ struct Engine {
   uint32_t wait_limit = kStreamWaitLimit;  // polls per mbarrier wait of the streaming kernel
   int withhold = -1;                       // test hook: plane the TMA kernels' producers never issue
   bool use_graph = true;  // replay the time loop as a captured CUDA graph
+  int direct_nt = -1;     // steps of the last run whose launches came from the host
   double last_ms = 0;
   double tune_ms = 0;      // host time of the autotuner's trial runs in the last tiling (0: cached choice)
   int tune_trials = 0;     // candidate shapes it timed
@@ -583,7 +584,7 @@ struct Engine {
   void reset_graph() {
     if (graph) cudaGraphExecDestroy(graph);
     graph = nullptr;
-    graph_nt = -1;
+    graph_nt = direct_nt = -1;
   }
 
   void build_tiles() {
@@ -1896,10 +1897,16 @@ struct Engine {
   void run_async(int nt) {
     init();
     cudaStream_t st = stream();
-    if (!use_graph) {  // every launch issued from the host, step by step
+    // A time loop's first run is launched from the host, its repetitions replay a
+    // graph. Making a graph, launching it the first time and destroying it costs
+    // about 5.5 us of host time per node and the GPU waits for it; a launch costs
+    // 2 us beside the steps before it (1500 half steps of 120x100x64 cells: 14 ms
+    // before the first step and 3 ms at the end, then 27 ms of steps).
+    if (!use_graph || (graph_nt != nt && direct_nt != nt)) {
       reset_graph();
       build_caps();
       uploads_done();
+      if (use_graph) direct_nt = nt;
       CK(cudaEventRecord(ev0, st));
       enqueue(st, nt);
       CK(cudaEventRecord(ev1, st));
