@@ -69,6 +69,22 @@ struct RowEq {
 };
 using RowMap = std::unordered_map<Row, uint32_t, RowHash, RowEq>;
 
+// d[z] = 0 where the coefficients of the n cells from `at` equal those of the
+// cells from `ref` bit for bit.
+__attribute__((target_clones("avx512f", "avx2", "default")))
+void column_differences(const float* const* coef, int64_t at, int64_t ref, int n, uint32_t* d) {
+  typedef uint32_t __attribute__((may_alias)) word;
+  for (int z = 0; z < n; ++z) d[z] = 0;
+  for (int c = 0; c < kNumCoef; c += 2) {
+    const word* a = reinterpret_cast<const word*>(coef[c] + at);
+    const word* b = reinterpret_cast<const word*>(coef[c] + ref);
+    const word* a2 = reinterpret_cast<const word*>(coef[c + 1] + at);
+    const word* b2 = reinterpret_cast<const word*>(coef[c + 1] + ref);
+    for (int z = 0; z < n; ++z) d[z] |= (a[z] ^ b[z]) | (a2[z] ^ b2[z]);
+  }
+}
+static_assert(kNumCoef % 2 == 0, "coefficient arrays are compared in pairs");
+
 }  // namespace
 
 GradedIndex::GradedIndex(const CompiledGrid& g, uint32_t mask) : nx(g.nx), ny(g.ny), nz(g.nz) {
@@ -302,15 +318,45 @@ bool compile_grid(int nx, int ny, int nz, const float* const* coef, const std::v
     Row prev;
     uint32_t prev_id = UINT32_MAX;
     std::vector<uint32_t> prev_col(static_cast<size_t>(nz), UINT32_MAX);  // ids of the previous (x, y) column
-    int64_t n_esplit = 0, n_hsplit = 0;
+    std::vector<uint32_t> diff[2] = {std::vector<uint32_t>(static_cast<size_t>(nz)),
+                                     std::vector<uint32_t>(static_cast<size_t>(nz))};
     // next probe cell at or after this slab's first cell
     size_t pc = size_t(std::lower_bound(probe_cells.begin(), probe_cells.end(), int64_t(xa) * ny * nz,
                                         [](const auto& a, int64_t c) { return a.first < c; }) -
                        probe_cells.begin());
     for (int x = xa; x < xb; ++x)
-      for (int y = 0; y < ny; ++y)
+      for (int y = 0; y < ny; ++y) {
+        // Most cells have the coefficients of their neighbour at y - 1, or at
+        // x - 1 (in a y layer): whole columns are compared, and a row is built
+        // only where both differ. The neighbour's row holds where the rules below
+        // for the last x plane and the last y row treat both cells alike. (Per
+        // cell 30 strided loads and a row: 120x100x64 cells 5.1 ms on 16 cores,
+        // 72x64x64 2.2 ms; compared by columns 3.9 and 1.5 ms, most of it memory.)
+        const int64_t col = (int64_t(x) * ny + y) * nz;
+        int64_t ref[2] = {-1, -1};
+        if (y > 0 && y < ny - 1) ref[0] = col - nz;
+        if (x > xa && x < nx - 1) ref[1] = col - int64_t(ny) * nz;
+        bool found = false;  // every cell of the column has an equal neighbour
+        for (int k = 0; k < 2 && !found; ++k) {
+          if (ref[k] < 0) continue;
+          column_differences(coef, col, ref[k], nz, diff[k].data());
+          found = std::all_of(diff[k].begin(), diff[k].end(), [](uint32_t d) { return d == 0; });
+          if (k == 0 && found) ref[1] = -1;
+        }
         for (int z = 0; z < nz; ++z) {
-          const int64_t cell = (int64_t(x) * ny + y) * nz + z;
+          const int64_t cell = col + z;
+          if (pc >= probe_cells.size() || probe_cells[pc].first != cell) {
+            uint32_t same = UINT32_MAX;
+            for (int k = 0; k < 2 && same == UINT32_MAX; ++k)
+              if (ref[k] >= 0 && diff[k][size_t(z)] == 0) {
+                const uint32_t id = local_ids[size_t(ref[k] + z)];
+                if ((rows[id].w[R_FLAGS] >> 16) == 0) same = id;  // (a probe cell's row is its own)
+              }
+            if (same != UINT32_MAX) {
+              prev_col[size_t(z)] = local_ids[size_t(cell)] = same;
+              continue;
+            }
+          }
           Row r;
           for (int c = 0; c < kNumCoef; ++c) r.w[kSlotOf[c]] = fbits(coef[c][cell]);
           if (x == nx - 1)  // solver_init_fields zeroes the last x plane of Cy, Cz, Dx
@@ -352,8 +398,6 @@ bool compile_grid(int nx, int ny, int nz, const float* const* coef, const std::v
           if (flags & (0x38u * kFlagCompSplit0)) flags |= kFlagHSplit;
           if (e_diff || h_diff) flags |= kFlagGraded;
           flags |= uint32_t(probe_count) << 16;
-          n_esplit += (flags & kFlagESplit) ? 1 : 0;  // thread-local: the shared counters sit in one cache line
-          n_hsplit += (flags & kFlagHSplit) ? 1 : 0;
           r.w[R_FLAGS] = flags;
           r.w[R_PROBE] = uint32_t(probe_first);
           // the row is usually that of the cell below (z - 1) or of the cell
@@ -380,8 +424,7 @@ bool compile_grid(int nx, int ny, int nz, const float* const* coef, const std::v
           prev_col[size_t(z)] = id;
           local_ids[size_t(cell)] = id;
         }
-    e_split[t] = n_esplit;
-    h_split[t] = n_hsplit;
+      }
   };
   {
     std::vector<std::thread> pool;
@@ -425,7 +468,20 @@ bool compile_grid(int nx, int ny, int nz, const float* const* coef, const std::v
       const int xb = xa + base + (t < rem ? 1 : 0);
       pool.emplace_back([&, t, xa, xb] {
         const size_t a = size_t(xa) * ny * nz, b = size_t(xb) * ny * nz;
-        for (size_t c = a; c < b; ++c) out.ids[c] = uint16_t(remap[t][local_ids[c]]);
+        std::vector<uint32_t> word(remap[t].size());  // row | E split | H split of each local row
+        for (size_t i = 0; i < word.size(); ++i) {
+          const uint32_t f = local_rows[t][i].w[R_FLAGS];
+          word[i] = remap[t][i] | (f & kFlagESplit ? 1u << 30 : 0u) | (f & kFlagHSplit ? 1u << 31 : 0u);
+        }
+        int64_t n_e = 0, n_h = 0;  // (the shared counters sit in one cache line)
+        for (size_t c = a; c < b; ++c) {
+          const uint32_t w = word[local_ids[c]];
+          out.ids[c] = uint16_t(w);
+          n_e += w >> 30 & 1u;
+          n_h += w >> 31;
+        }
+        e_split[t] = n_e;
+        h_split[t] = n_h;
       });
       xa = xb;
     }
