@@ -97,6 +97,7 @@ struct StreamGeom {
   static constexpr int XCH = 2 * ER * 32 * 4;      // one E neighbour-exchange buffer (ex, ez), bytes
   // resident blocks per SM the register budget is sized for (shared memory allows as many)
   static constexpr int MIN_BLOCKS = TY <= 4 ? 4 : TY <= 6 ? 3 : 2;
+  static constexpr int PLAIN_BLOCKS = TY <= 4 ? 5 : TY <= 6 ? 4 : TY <= 8 ? 3 : 2;  // of kTilesPlainMost
 };
 
 // Plane slots and split regions of the streaming kernel (at most). A plane
@@ -157,16 +158,21 @@ __device__ __forceinline__ void stream_inject(const SimDev& Sd, const float4& r7
   }
 }
 
-// PLAIN_ONLY: an instantiation for lists of plain tiles only, compiled
-// with the interior plane loop alone (fewer live registers, no split
-// regions); it runs beside the general instantiation, which takes the tiles
-// with split-field or probe cells.
-template <int TY, bool PLAIN_ONLY>
-__global__ void __launch_bounds__(StreamGeom<TY>::THREADS, StreamGeom<TY>::MIN_BLOCKS)
-fdtd_step_stream_kernel(const SimDev* __restrict__ sims, const StreamTile* __restrict__ tiles, int n_tiles, int n,
+// TILES: kTilesAny takes tiles with split-field or probe cells. kTilesPlain is
+// for lists of plain tiles only, compiled with the interior plane loop alone
+// (fewer live registers, no split regions), and runs beside it; kTilesPlainMost
+// is the same with registers for more blocks per SM, for grids of almost only
+// plain tiles. ONE: a single simulation, whose descriptor is a kernel parameter
+// (a load from global memory per use in the plane loop otherwise).
+enum { kTilesAny, kTilesPlain, kTilesPlainMost };
+
+template <int TY, int TILES, bool ONE>
+__global__ void __launch_bounds__(StreamGeom<TY>::THREADS, TILES == kTilesPlainMost ? StreamGeom<TY>::PLAIN_BLOCKS : StreamGeom<TY>::MIN_BLOCKS)
+fdtd_step_stream_kernel(const __grid_constant__ SimDev one, const SimDev* __restrict__ sims, const StreamTile* __restrict__ tiles, int n_tiles, int n,
                         unsigned* __restrict__ counter, unsigned base, int* __restrict__ err, int n_main,
                         int n_reg, uint32_t wait_limit, int withhold) {
   using G = StreamGeom<TY>;
+  constexpr bool PLAIN_ONLY = TILES != kTilesAny;
   // dynamic shared memory: the E exchange buffers, n_main plane slots (H, E,
   // index), n_reg split regions (E and H pairs of one slab store). A warp
   // holds two plane slots (the plane and its look-ahead) and their regions at
@@ -225,9 +231,10 @@ fdtd_step_stream_kernel(const SimDev* __restrict__ sims, const StreamTile* __res
         td = load_stream_tile(tiles, t);
         nload = td.z1 - td.z0 + 2;  // planes z0-1 .. z1
         mask = uint64_t(td.split_lo) | (uint64_t(td.split_hi) << 32);
-        maps = reinterpret_cast<const StreamMaps*>(sims[td.sim].maps);
-        sp = &sims[td.sim].sp;
-        snz = sims[td.sim].nz;
+        const SimDev& Sp = ONE ? one : sims[td.sim];
+        maps = reinterpret_cast<const StreamMaps*>(Sp.maps);
+        sp = &Sp.sp;
+        snz = Sp.nz;
         if (maps != cur_maps) {
           tensormap_acquire(&maps->E);
           tensormap_acquire(&maps->H);
@@ -346,7 +353,7 @@ fdtd_step_stream_kernel(const SimDev* __restrict__ sims, const StreamTile* __res
     const int ti = s_tq[k & 3];
     if (ti < 0) break;
     const StreamTile td = load_stream_tile(tiles, ti);
-    const SimDev& Sd = sims[td.sim];
+    const SimDev& Sd = ONE ? one : sims[td.sim];
     const int x0 = td.x0, y0 = td.y0, z0 = td.z0;
     const int c = x0 - 1 + lane, r = y0 - 1 + w;
     const int oh = (x0 - 1) - ((x0 - 1) & ~3), oi = (x0 - 1) - ((x0 - 1) & ~7);
