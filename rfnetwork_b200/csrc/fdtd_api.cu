@@ -831,7 +831,7 @@ struct Engine {
 
   // Blocks over every cell of every simulation, of the size around `want`
   // threads that leaves the fewest idle over all grids; returns that size.
-  int half_blocks(int want, std::vector<int4>& blocks) const {
+  int half_blocks(int want, std::vector<int4>& blocks, int deep = 1) const {
     double best = -1.0;
     int threads = want;
     for (int t = std::max(64, want / 2); t <= kHalfThreads; t += 32) {
@@ -851,7 +851,7 @@ struct Engine {
       const fdtd_sim* s = sims[i];
       int seg, rows;
       half_shape(s->nx, s->ny, threads, &seg, &rows);
-      for (int z = 0; z < s->nz; ++z)
+      for (int z = 0; z < s->nz; z += deep)
         for (int y0 = 0; y0 < s->ny; y0 += rows)
           for (int x0 = 0; x0 < s->nx; x0 += seg)
             blocks.push_back(make_int4(int(i), x0 | (rows << 16), y0, z | (seg << 16)));
@@ -1633,14 +1633,21 @@ struct Engine {
     dim3 half_grid;
     int half_threads = 0;
     if (half_adj) {
+      // Cells per thread along z: rows are read less often, but a small grid runs
+      // out of threads. 200 steps forward and back with 1 / 2 / 4 cells: 52x44x33
+      // 4.55 / 5.82 / 7.95 ms, 80x72x60 8.05 / 8.21 / 9.67, 96x96x64 11.71 / 11.16 /
+      // 12.09, 128x128x96 25.85 / 23.42 / 22.68, 160x150x120 49.92 / 46.83 / 45.81.
+      int64_t cells = 0;
+      for (const auto& a : as) cells += int64_t(a.nx) * a.ny * a.nz;
+      hl.deep = cells < 400'000 ? 1 : cells < 1'000'000 ? 2 : 4;
       if (as.size() == 1) {
         half_shape(as[0].nx, as[0].ny, kAdjHalfWant, &hl.seg, &hl.rows);
         half_threads = (hl.seg * hl.rows + 31) / 32 * 32;
         half_grid = dim3(unsigned((as[0].nx + hl.seg - 1) / hl.seg), unsigned((as[0].ny + hl.rows - 1) / hl.rows),
-                         unsigned(as[0].nz));
+                         unsigned((as[0].nz + hl.deep - 1) / hl.deep));
       } else {
         std::vector<int4> blocks;
-        half_threads = half_blocks(kAdjHalfWant, blocks);
+        half_threads = half_blocks(kAdjHalfWant, blocks, hl.deep);
         half_grid = dim3(unsigned(blocks.size()));
         adj_d_blocks.reserve(blocks.size());
         CK(cudaMemcpy(adj_d_blocks.p, blocks.data(), blocks.size() * sizeof(int4), cudaMemcpyHostToDevice));

@@ -51,6 +51,7 @@ struct HalfLaunch {
   int seg, rows, planes;
   int lo, hi;
   int n;                 // time step
+  int deep;              // reverse step: planes per block
 };
 
 struct HalfPlace {

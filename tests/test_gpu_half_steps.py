@@ -135,3 +135,22 @@ def test_batched_gradients_equal_single(engine_lib, monkeypatch):
     assert all(np.abs(w).max() > 0 for w in want)
     for got in out.values():
         assert all(np.array_equal(x, y) for x, y in zip(got, want))
+
+
+# grids large enough for two and four cells per thread along z, with a remainder
+@pytest.mark.parametrize("sizes", [[(90, 80, 59)], [(120, 110, 77)], [(90, 80, 59), (92, 70, 61)]])
+def test_gradients_of_deep_columns(engine_lib, monkeypatch, sizes):
+    nt, out = 50, []
+    models = [configs.microstrip(n=n, n_pml=5, nt=nt) for n in sizes]
+    boxes = [(n[0] // 2 - 4, n[0] // 2 + 5, n[1] // 2 - 3, n[1] // 2 + 6, 8, 12) for n in sizes]
+    monkeypatch.setenv("RFN_FDTD_KERNEL", "half")  # (members of a batch step together)
+    for half in ("1", "0"):
+        monkeypatch.setenv("RFN_ADJ_HALF", half)
+        sims = [_model_sim(s)[0] for s in models]
+        b = _lib.Batch(sims)
+        b.run_recorded(nt, boxes)
+        out.append(b.adjoint([2 * sim.dft() for sim in sims]))
+        b.close()
+        for sim in sims:
+            sim.close()
+    assert all(np.abs(g).max() > 0 and np.array_equal(g, w) for g, w in zip(*out))
