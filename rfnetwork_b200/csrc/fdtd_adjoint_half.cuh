@@ -14,7 +14,7 @@
 // along z they change only at the model's and the z layers' boundaries, so a
 // thread keeps them while the four ids stay the same. 128x128x96 cells with
 // 10-cell layers, per step: one launch 89 us, halves of one cell per thread 71,
-// of four 55; small grids need every thread. 80 registers and 24 warps
+// of four 65; small grids need every thread. 80 registers and 24 warps
 // per SM instead of 64 and 32 lose 5 %; halves kept per component instead of per
 // cell move a third less in the layers and were slower (more branches per
 // access). The arithmetic and its roundings are those of adj_e_part and

@@ -146,7 +146,8 @@ struct KernelConfig {
                     // half steps: threads per block
   int stages = 6;   // streaming: shared-memory plane slots; resident: bricks along y
   int zchunk = 0;   // 0: pick from the grid size; resident: bricks along z
-  int one_list = 0; // streaming: every tile through the general instantiation (no plain-tile kernel beside it)
+  int one_list = 0; // streaming: every tile through the general instantiation (no plain-tile kernel beside it);
+                    // resident: weight of a layer's plane, percent of another's
 };
 
 // Step-kernel shapes the autotuner times, (variant, tile height, plane slots,
@@ -666,28 +667,90 @@ struct Engine {
     return sims.size() == 1 && sims[0]->adj_mode == 0;
   }
 
-  // Partitions (bricks along x, y, z) worth timing, the cheapest first per
-  // number of blocks: the largest brick's cells and face cells bound a step.
-  // None when the grid's fields alone exceed the shared memory.
-  std::vector<std::array<int, 3>> resident_partitions(int n_sm) const {
-    std::vector<std::array<int, 3>> out;
-    const fdtd_sim* s = sims[0];
-    for (const int most : {n_sm, n_sm / 2, 32, 8}) {
-      double best = 1e300;
-      std::array<int, 3> pick{0, 0, 0};
-      for (int px = 1; px <= std::min(most, s->nx); ++px)
-        for (int py = 1; px * py <= most && py <= s->ny; ++py)
-          for (int pz = 1; px * py * pz <= most && pz <= s->nz; ++pz) {
-            const int bx = (s->nx + px - 1) / px, by = (s->ny + py - 1) / py, bz = (s->nz + pz - 1) / pz;
-            if (res_smem(bx, by, bz, 0) > kResSmemMax) continue;
-            const double cost = double(bx) * by * bz + 0.75 * (double(bx) * by + double(bx) * bz + double(by) * bz);
-            if (cost < best) {
-              best = cost;
-              pick = {px, py, pz};
-            }
-          }
-      if (pick[0] && std::find(out.begin(), out.end(), pick) == out.end()) out.push_back(pick);
+  // The cuts of a simulation into px x py x pz bricks, a cell plane of a layer
+  // weighing `weight` percent of another; false when a brick would be empty.
+  static bool resident_cuts(const fdtd_sim* s, int px, int py, int pz, int weight, ResPart& P) {
+    const int n[3] = {s->nx, s->ny, s->nz}, parts[3] = {px, py, pz};
+    P.px = px; P.py = py; P.pz = pz;
+    for (int a = 0; a < 3; ++a) {
+      if (parts[a] >= kResCuts || parts[a] > n[a]) return false;
+      const int64_t lo = s->split_plan.t[2 * a], hi = s->split_plan.t[2 * a + 1], mid = n[a] - lo - hi;
+      const int64_t wl = lo * weight, wm = mid * 100, all = wl + wm + hi * weight;
+      P.most[a] = 0;
+      for (int i = 0; i <= parts[a]; ++i) {
+        // the first cell whose planes below weigh i / parts of all (the layers' weights cancel at 100)
+        const int64_t w = all * i / parts[a];
+        const int64_t c = w <= wl ? w / weight : w <= wl + wm ? lo + (w - wl) / 100 : lo + mid + (w - wl - wm) / weight;
+        P.cut[a][i] = uint16_t(i == parts[a] ? n[a] : c);
+        if (i > 0) {
+          if (P.cut[a][i] <= P.cut[a][i - 1]) return false;
+          P.most[a] = std::max(P.most[a], int(P.cut[a][i]) - int(P.cut[a][i - 1]));
+        }
+      }
     }
+    return true;
+  }
+
+  // Partitions worth timing, (bricks along x, y, z, weight): per number of blocks
+  // the one whose costliest brick costs least, with even cuts and with thinner
+  // bricks in the layers. A brick's cost: its cells, 0.7 more per layer cell,
+  // 0.75 per face cell; its memory from the layers the split plan found. None when no
+  // partition fits. Thinner bricks take grids that even cuts do not (125x46x86
+  // cells with 8-cell layers: half steps 14.0, here 10.7 us per step; 133x44x88
+  // 15.5 -> 11.4) and even out the time (55x140x47 8.6 -> 8.0 us).
+  std::vector<std::array<int, 4>> resident_partitions(int n_sm) const {
+    std::vector<std::array<int, 4>> out;
+    const fdtd_sim* s = sims[0];
+    const int n[3] = {s->nx, s->ny, s->nz};
+    const int* t = s->split_plan.t;
+    struct Part { int len, layer; };  // cells of a brick along an axis, of these in a layer
+    auto cost_of = [&](const ResPart& P) -> double {
+      std::vector<Part> kinds[3];
+      const int parts[3] = {P.px, P.py, P.pz};
+      for (int a = 0; a < 3; ++a)
+        for (int i = 0; i < parts[a]; ++i) {
+          const int c0 = P.cut[a][i], c1 = P.cut[a][i + 1];
+          const int layer = std::max(0, std::min(c1, t[2 * a]) - c0) + std::max(0, c1 - std::max(c0, n[a] - t[2 * a + 1]));
+          bool seen = false;
+          for (const auto& k : kinds[a]) seen = seen || (k.len >= c1 - c0 && k.layer >= layer);
+          if (!seen) kinds[a].push_back({c1 - c0, layer});
+        }
+      double worst = 0;
+      for (const auto& x : kinds[0])
+        for (const auto& y : kinds[1])
+          for (const auto& z : kinds[2]) {
+            const int v = x.len * y.len * z.len;
+            auto either = [](const Part& p, const Part& q) { return p.len * q.len - (p.len - p.layer) * (q.len - q.layer); };
+            const int pairs = 2 * (x.len * either(y, z) + y.len * either(x, z) + z.len * either(x, y));
+            if (res_smem(x.len, y.len, z.len, pairs) > kResSmemMax) return 1e300;
+            const int core = (x.len - x.layer) * (y.len - y.layer) * (z.len - z.layer);
+            worst = std::max(worst, v + 0.7 * (v - core) + 0.75 * (x.len * y.len + x.len * z.len + y.len * z.len));
+          }
+      return worst;
+    };
+    const bool layers = t[0] + t[1] + t[2] + t[3] + t[4] + t[5] > 0;
+    ResPart P;
+    for (const int most : {n_sm, n_sm / 2, 32, 8})
+      for (const int thin : {0, 1}) {
+        if (thin && (!layers || most != n_sm)) continue;
+        double best = 1e300;
+        std::array<int, 4> pick{0, 0, 0, 0};
+        for (int px = 1; px <= std::min(most, s->nx); ++px)
+          for (int py = 1; px * py <= most && py <= s->ny; ++py)
+            for (int pz = 1; px * py * pz <= most && pz <= s->nz; ++pz) {
+              // (with fewer than three quarters of the blocks the next smaller `most` is at hand)
+              if (4 * px * py * pz < 3 * most && most <= s->nx * s->ny * s->nz / 64) continue;
+              for (const int w : {100, 125, 150}) {
+                if ((w == 100) == (thin == 1) || !resident_cuts(s, px, py, pz, w, P)) continue;
+                const double cost = cost_of(P);
+                if (cost < best) {
+                  best = cost;
+                  pick = {px, py, pz, w};
+                }
+              }
+            }
+        if (pick[0] && std::find(out.begin(), out.end(), pick) == out.end()) out.push_back(pick);
+      }
     return out;
   }
 
@@ -697,8 +760,10 @@ struct Engine {
     ResidentClass& c = res;
     fdtd_sim* s = sims[0];
     const int px = cfg.ty, py = cfg.stages, pz = cfg.zchunk, nb = px * py * pz;
+    ResPart& P = c.g.part;
     if (nb > n_sm) throw ArgError{FDTD_ERR_LIMIT, "More bricks than SMs."};
-    const int bx = (s->nx + px - 1) / px, by = (s->ny + py - 1) / py, bz = (s->nz + pz - 1) / pz;
+    if (!resident_cuts(s, px, py, pz, cfg.one_list, P)) throw ArgError{FDTD_ERR_LIMIT, "More bricks than cells."};
+    const int bx = P.most[0], by = P.most[1], bz = P.most[2];
     const int cells = bx * by * bz, nf = 2 * (by * bz + bx * bz + bx * by);
     if (ResBox{0, 0, 0, bx, by, bz, 0, 0, 0}.size() * int64_t(3) >= kResNone || res_smem(bx, by, bz, 0) > kResSmemMax)
       throw ArgError{FDTD_ERR_LIMIT, "Bricks do not fit in shared memory."};
@@ -710,16 +775,17 @@ struct Engine {
     n_nums.alloc(size_t(nb));
     const ResScratch scratch{map.p, nums.p, n_rows, cells};
     CK(cudaMemset(map.p, 0xff, map.n * sizeof(int)));
-    res_count_kernel<<<nb, 32>>>(s->dev, px, py, pz, scratch, c.count.p, n_nums.p);
+    res_count_kernel<<<nb, 32>>>(s->dev, P, scratch, c.count.p, n_nums.p);
     CK(cudaGetLastError());
     std::vector<int4> cnt(static_cast<size_t>(nb));
     CK(cudaMemcpy(cnt.data(), c.count.p, cnt.size() * sizeof(int4), cudaMemcpyDeviceToHost));
-    int pairs = 0, local = 0;
-    for (const auto& k : cnt) {
-      pairs = std::max(pairs, k.z);
-      local = std::max(local, k.w);
+    int local = 0;
+    uint32_t state = 0;
+    for (int b = 0; b < nb; ++b) {
+      const ResBox r = res_box(P, b);
+      state = std::max(state, res_smem(r.bx, r.by, r.bz, cnt[size_t(b)].z));
+      local = std::max(local, cnt[size_t(b)].w);
     }
-    const uint32_t state = res_smem(bx, by, bz, pairs);
     if (state > kResSmemMax) throw ArgError{FDTD_ERR_LIMIT, "Bricks do not fit in shared memory."};
     const int row_cap = std::min<int>(local, int((kResSmemMax - state) / kResRowBytes));
     c.smem = state + uint32_t(row_cap) * kResRowBytes;
@@ -730,7 +796,6 @@ struct Engine {
     c.face.alloc(size_t(2) * nb * nf);
     ResGrid& g = c.g;
     g.s = s->dev;
-    g.px = px; g.py = py; g.pz = pz;
     g.cap = cells;
     g.row_cap = row_cap;
     g.e_list = c.lists.p;
@@ -754,7 +819,7 @@ struct Engine {
       int most_el = 1;
       for (int b = 0; b < nb; ++b) {
         int el = 0;
-        for (const auto& m : mons) el += res_mon_elements(m, res_box(s->dev, px, py, pz, b));
+        for (const auto& m : mons) el += res_mon_elements(m, res_box(P, b));
         most_el = std::max(most_el, el);
       }
       c.mon_list.alloc(size_t(nb) * most_el);
@@ -771,10 +836,10 @@ struct Engine {
         c.smem += uint32_t(g.acc_cap) * 8u * uint32_t(g.acc_f);
       }
       g.mon_count = c.mon_count.p;
-      res_monitor_kernel<<<nb, 128>>>(s->dev, px, py, pz, s->d_mons.p, g.n_mon, most_el, c.mon_list.p, c.mon_count.p);
+      res_monitor_kernel<<<nb, 128>>>(P, s->d_mons.p, g.n_mon, most_el, c.mon_list.p, c.mon_count.p);
       CK(cudaGetLastError());
     }
-    res_build_kernel<<<nb, 32>>>(s->dev, px, py, pz, scratch, n_nums.p, cells, row_cap, c.lists.p, c.lists.p + nl,
+    res_build_kernel<<<nb, 32>>>(s->dev, P, scratch, n_nums.p, cells, row_cap, c.lists.p, c.lists.p + nl,
                                  c.lists.p + 2 * nl, c.lists.p + 3 * nl, c.row_ids.p, c.stride.p);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(0));
@@ -960,24 +1025,26 @@ struct Engine {
     tune_trials = 0;
     if (resident_allowed()) {
       std::vector<TuneChoice> cand;
-      for (const auto& p : resident_partitions(n_sm)) cand.push_back({2, p[0], p[1], p[2], 0});
-      if (!cand.empty() && tune(n_sm, cand, 2)) return;
+      if (tune(n_sm, cand, 2)) return;
     }
     std::vector<TuneChoice> cand;
     for (const auto& c : kTuneCandidates) cand.push_back({c[0], c[1], c[2], c[3], c[4]});
     tune(n_sm, cand, 1);
   }
 
-  // Times the candidates (all of one kernel) and builds the best one; false
-  // when none fits.
-  bool tune(int n_sm, const std::vector<TuneChoice>& cand, int variant) {
+  // Times the candidates (given, or the resident kernel's partitions) and builds
+  // the best one; false when none fits.
+  bool tune(int n_sm, const std::vector<TuneChoice>& given, int variant) {
     std::vector<int> key{variant};
     int nt_min = 1 << 30;
     for (auto* s : sims) {
       key.insert(key.end(), {s->nx, s->ny, s->nz});
       nt_min = std::min(nt_min, s->prepared_nt);
     }
+    // (what fits in shared memory depends on the layers)
+    if (variant == 2) key.insert(key.end(), sims[0]->split_plan.t, sims[0]->split_plan.t + 6);
     const KernelConfig auto_cfg = cfg;
+    std::vector<TuneChoice> cand = given;
     auto build = [&](const TuneChoice& c) -> bool {
       cfg.variant = c[0];
       cfg.ty = c[1];
@@ -1003,7 +1070,10 @@ struct Engine {
         best = it->second;
       }
     }
+    if (cached && best[0] < 0) return false;  // nothing fitted
     if (cached && build(best)) return true;  // (a model of the same size may hold more split cells)
+    if (variant == 2)
+      for (const auto& p : resident_partitions(n_sm)) cand.push_back({2, p[0], p[1], p[2], p[3]});
     // (a launch of the resident kernel also loads and stores the state)
     const int warm = 2, timed = std::min(variant == 2 ? 64 : 8, nt_min - warm);
     bool found = false;
@@ -1053,12 +1123,12 @@ struct Engine {
     }
     check_error();
     tune_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    if (!found) return false;
+    if (!found) best[0] = -1;
     {
       std::lock_guard<std::mutex> lock(g_tune_mutex);
       g_tune_cache[key] = best;
     }
-    return build(best);
+    return found && build(best);
   }
 
   // Streaming kernel: 31 x TY column tiles cut in z chunks of at most 62
@@ -1405,7 +1475,7 @@ struct Engine {
   DevBuf<unsigned> adj_counter;   // its tile counter
   DevBuf<int4> adj_d_blocks;      // half-step reverse: blocks over several simulations
   static constexpr int kAdjHalfWant = 128;                // its threads per block (64 and 256: up to 10 % slower)
-  static constexpr int64_t kAdjHalfBytes = 120'000'000;
+  static constexpr int64_t kAdjHalfBytes = 160'000'000;
   static int adj_tiles_per_sm() {
     const char* v = std::getenv("RFN_ADJ_TILES_PER_SM");
     return v ? std::max(1, std::atoi(v)) : 4;
@@ -1489,11 +1559,10 @@ struct Engine {
     // The half-step reverse where its state (six totals per cell, six halves more
     // per cell with split E or H) fits in L2, which then serves it twice per step;
     // beyond that one launch per step, which reads it once. Per step, one launch
-    // against two halves: 52x44x33 cells with 6-cell layers 20.5 against 12.7 us,
-    // 96x96x64 with 10 39.6 against 31.1, 128x128x96 with 10 (74 MB) 88.9 against
-    // 71.3, 160x150x120 with 6 (98 MB) 148.6 against 139.3; 224x200x128 with 8
-    // (195 MB) 247 against 259, and a design step of six 96x96x64 members (185 MB)
-    // 105 against 111 ms. RFN_ADJ_HALF=0 / 1 decides.
+    // against two halves: 52x44x33 cells with 6-cell layers 22.6 against 9.4 us,
+    // 96x96x64 with 10 39.6 against 29.8, 128x128x96 with 10 (75 MB) 88.8 against
+    // 64.7, 160x150x120 with 6 (101 MB) 148.6 against 136.2, 190x170x120 with 6 (133
+    // MB) 181 against 167; 224x200x128 with 8 (207 MB) 248 against 251. RFN_ADJ_HALF=0 / 1 decides.
     int64_t adj_state = 0;
     for (const auto& rq : req)
       adj_state += 24 * (int64_t(rq.s->nx) * rq.s->ny * rq.s->nz + rq.s->grid.e_split_cells + rq.s->grid.h_split_cells);

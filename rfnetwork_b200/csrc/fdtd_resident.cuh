@@ -7,7 +7,8 @@
 // keeps one brick of the grid in shared memory for the whole launch, so a step
 // is shared-memory arithmetic plus the exchange of the brick's faces.
 //
-//   brick     the grid is cut into px x py x pz bricks, one block each, all
+//   brick     the grid is cut into px x py x pz bricks (thinner ones in the
+//             absorbing layers where that pays), one block each, all
 //             resident at once (cooperative launch). E and H of the brick's
 //             cells and one halo layer (H above, E below) and the split pairs
 //             of its split cells live in shared memory
@@ -37,8 +38,9 @@
 // Measured on a B200, per step, against the streaming kernels' best shape (one
 // or two launches per step): 24x20x16 cells, 4-cell layers 9.0 -> 2.9 us;
 // 64x64x48, 10-cell layers 17.2 -> 5.6 us; 91x71x53 graded, 7-cell layers 20.6
-// -> 7.9 us; 100x80x64, 5-cell layers 25.8 -> 10.0 us; 120x110x80 without
-// layers (the largest that fits) 22.3 -> 16.3 us. What bounds it now is a
+// -> 7.7 us; 100x80x64, 5-cell layers 25.8 -> 9.5 us; 133x44x88, 8-cell layers
+// (about the most that fits with such layers) 11.4 us, half steps 15.5; 120x110x80
+// without layers 22.3 -> 16.0 us. What bounds it now is a
 // warp's chain of about a hundred dependent instructions per cell and phase
 // (about 700 cycles, two or three cells per thread), shared-memory wavefronts,
 // and two exchanges per step of about 0.6 us each, partly hidden. Two cells per
@@ -97,10 +99,20 @@ __device__ __forceinline__ void res_record(const SimDev& S, const float4& r7, in
   }
 }
 
+// How a grid is cut: bricks along each axis and the first cells of each. Layer
+// cells cost more time (two values and an addition per component) and memory
+// (up to 72 bytes instead of 24), so bricks in the layers may be thinner.
+constexpr int kResCuts = 152;       // most bricks along an axis, and one
+struct ResPart {
+  int px, py, pz;
+  int most[3];                     // cells of the longest brick along each axis
+  uint16_t cut[3][kResCuts];
+};
+
 // The partition and the lists of one simulation.
 struct ResGrid {
   SimDev s;
-  int px, py, pz;          // bricks along each axis
+  ResPart part;
   int cap;                 // list entries per brick
   int row_cap;             // most table rows a brick keeps in shared memory
   const uint2* e_list;     // [brick][cap]: cell | row << 16, pair slot | (split components, flags) << 16
@@ -122,9 +134,6 @@ struct ResGrid {
   uint32_t wait_limit;
 };
 
-// First cell of part i of n cells cut into p parts.
-__host__ __device__ __forceinline__ int res_cut(int n, int p, int i) { return int(int64_t(n) * i / p); }
-
 struct ResBox {
   int x0, y0, z0, bx, by, bz, ix, iy, iz;
   // strides of the brick's field arrays, which have one halo layer: odd, so that
@@ -134,17 +143,17 @@ struct ResBox {
   __host__ __device__ int size() const { return sz() * (bz + 1); }
 };
 
-__host__ __device__ __forceinline__ ResBox res_box(const SimDev& S, int px, int py, int pz, int b) {
+__host__ __device__ __forceinline__ ResBox res_box(const ResPart& P, int b) {
   ResBox r;
-  r.ix = b % px;
-  r.iy = (b / px) % py;
-  r.iz = b / (px * py);
-  r.x0 = res_cut(S.nx, px, r.ix);
-  r.y0 = res_cut(S.ny, py, r.iy);
-  r.z0 = res_cut(S.nz, pz, r.iz);
-  r.bx = res_cut(S.nx, px, r.ix + 1) - r.x0;
-  r.by = res_cut(S.ny, py, r.iy + 1) - r.y0;
-  r.bz = res_cut(S.nz, pz, r.iz + 1) - r.z0;
+  r.ix = b % P.px;
+  r.iy = (b / P.px) % P.py;
+  r.iz = b / (P.px * P.py);
+  r.x0 = P.cut[0][r.ix];
+  r.y0 = P.cut[1][r.iy];
+  r.z0 = P.cut[2][r.iz];
+  r.bx = P.cut[0][r.ix + 1] - r.x0;
+  r.by = P.cut[1][r.iy + 1] - r.y0;
+  r.bz = P.cut[2][r.iz + 1] - r.z0;
   return r;
 }
 
@@ -177,7 +186,7 @@ struct ResCell {
   int lx, ly, lz;
 };
 
-__device__ __forceinline__ ResCell res_cell(const SimDev& s, const ResBox& r, int px, int py, int pz, int c) {
+__device__ __forceinline__ ResCell res_cell(const SimDev& s, const ResPart& P, const ResBox& r, int c) {
   ResCell q;
   q.lx = c % r.bx;
   q.ly = (c / r.bx) % r.by;
@@ -185,9 +194,9 @@ __device__ __forceinline__ ResCell res_cell(const SimDev& s, const ResBox& r, in
   q.id = s.mat[(r.z0 + q.lz) * s.plane + (r.y0 + q.ly) * s.pitch + r.x0 + q.lx];
   q.flags = __float_as_uint(s.rows[8 * q.id + 7].z);
   q.k = q.lz * r.sz() + q.ly * r.sy() + q.lx;
-  q.ex = q.lx == r.bx - 1 && r.ix + 1 < px;
-  q.ey = q.ly == r.by - 1 && r.iy + 1 < py;
-  q.ez = q.lz == r.bz - 1 && r.iz + 1 < pz;
+  q.ex = q.lx == r.bx - 1 && r.ix + 1 < P.px;
+  q.ey = q.ly == r.by - 1 && r.iy + 1 < P.py;
+  q.ez = q.lz == r.bz - 1 && r.iz + 1 < P.pz;
   q.hx = q.lx == 0 && r.ix > 0;
   q.hy = q.ly == 0 && r.iy > 0;
   q.hz = q.lz == 0 && r.iz > 0;
@@ -212,10 +221,10 @@ __device__ __forceinline__ int res_take(int* n, int key, unsigned on) {
 // in the order they appear, gives those that may be local a place in the local
 // table, and counts the cells of each row, the pairs and the face cells.
 __global__ void __launch_bounds__(32)
-res_count_kernel(const SimDev s, int px, int py, int pz, const ResScratch X, int4* __restrict__ count,
+res_count_kernel(const SimDev s, const __grid_constant__ ResPart P, const ResScratch X, int4* __restrict__ count,
                  int* __restrict__ n_nums) {
   const int lane = threadIdx.x, b = blockIdx.x;
-  const ResBox r = res_box(s, px, py, pz, b);
+  const ResBox r = res_box(P, b);
   const int cells = r.bx * r.by * r.bz;
   int* const mp = X.map + size_t(b) * X.n_rows;
   int* const info = X.of(b, 0);
@@ -224,7 +233,7 @@ res_count_kernel(const SimDev s, int px, int py, int pz, const ResScratch X, int
     const int c = c0 + lane;
     const unsigned on = __ballot_sync(0xffffffffu, c < cells);
     if (c < cells) {
-      const ResCell q = res_cell(s, r, px, py, pz, c);
+      const ResCell q = res_cell(s, P, r, c);
       const bool ef = q.ex || q.ey || q.ez, hf = q.hx || q.hy || q.hz;
       fe += ef;
       fh += hf;
@@ -270,19 +279,19 @@ res_count_kernel(const SimDev s, int px, int py, int pz, const ResScratch X, int
 // Second pass: the lists of one brick (one warp), ordered by face cell or not,
 // then by set of split components, then by table row.
 __global__ void __launch_bounds__(32)
-res_build_kernel(const SimDev s, int px, int py, int pz, const ResScratch X, const int* __restrict__ n_nums, int cap,
+res_build_kernel(const SimDev s, const __grid_constant__ ResPart P, const ResScratch X, const int* __restrict__ n_nums, int cap,
                  int row_cap, uint2* __restrict__ e_list, uint2* __restrict__ h_list, uint2* __restrict__ e_words,
                  uint2* __restrict__ h_words, uint16_t* __restrict__ row_ids, uint16_t* __restrict__ stride) {
   __shared__ int n_m[64];
   const int lane = threadIdx.x, b = blockIdx.x;
-  const ResBox r = res_box(s, px, py, pz, b);
+  const ResBox r = res_box(P, b);
   const int cells = r.bx * r.by * r.bz, nums = n_nums[b];
   const int* const mp = X.map + size_t(b) * X.n_rows;
   const int* const info = X.of(b, 0);
   int* const order = X.of(b, 6);
   // first words of the y and z faces (laid out for the largest brick, so that
   // a face has the same words in both bricks' buffers)
-  const int mx = (s.nx + px - 1) / px, my = (s.ny + py - 1) / py, mz = (s.nz + pz - 1) / pz;
+  const int mx = P.most[0], my = P.most[1], mz = P.most[2];
   const int wy = 2 * my * mz, wz = wy + 2 * mx * mz;
   auto split_set = [&](int k) { return int((__float_as_uint(s.rows[8 * (info[k] & 0xffff) + 7].z) >> 8) & 63u); };
   // the numbers in order of their split sets (most components first)
@@ -361,7 +370,7 @@ res_build_kernel(const SimDev s, int px, int py, int pz, const ResScratch X, con
     const int c = c0 + lane;
     const unsigned on = __ballot_sync(0xffffffffu, c < cells);
     if (c < cells) {
-      const ResCell q = res_cell(s, r, px, py, pz, c);
+      const ResCell q = res_cell(s, P, r, c);
       const bool ef = q.ex || q.ey || q.ez, hf = q.hx || q.hy || q.hz;
       const int k = mp[q.id];
       const int tab = int(unsigned(info[k]) >> 16);
@@ -400,9 +409,9 @@ __host__ __device__ __forceinline__ int res_mon_elements(const MonDev& M, const 
 // Lists the monitor elements of one brick (one block), monitor by monitor, in
 // the order of the monitor's output.
 __global__ void __launch_bounds__(128)
-res_monitor_kernel(const SimDev s, int px, int py, int pz, const MonDev* __restrict__ mons, int n_mon, int cap,
+res_monitor_kernel(const __grid_constant__ ResPart P, const MonDev* __restrict__ mons, int n_mon, int cap,
                    uint2* __restrict__ list, int* __restrict__ count) {
-  const ResBox r = res_box(s, px, py, pz, blockIdx.x);
+  const ResBox r = res_box(P, blockIdx.x);
   const int e0 = 1 + r.sy() + r.sz();
   int base = 0;
   for (int m = 0; m < n_mon; ++m) {
@@ -454,7 +463,7 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
   __shared__ int s_sample[MON ? kResMonitors : 1];  // this step's sample of each monitor, -1: none
   const SimDev& S = G.s;
   const int T = blockDim.x, tid = threadIdx.x;
-  const ResBox r = res_box(S, G.px, G.py, G.pz, blockIdx.x);
+  const ResBox r = res_box(G.part, blockIdx.x);
   // Position k = (lz, ly, lx) of own cell (lx, ly, lz). The three components of
   // a position lie side by side: the three words' odd stride keeps a warp's
   // accesses free of bank conflicts and a neighbour costs one address. H has
@@ -552,7 +561,7 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
     const int fx = r.by * r.bz, fy = r.bx * r.bz, fz = r.bx * r.by;
     // words of the x, y and z faces, laid out for the largest brick so that a
     // face has the same words in both bricks' buffers
-    const int mx = (S.nx + G.px - 1) / G.px, my = (S.ny + G.py - 1) / G.py, mz = (S.nz + G.pz - 1) / G.pz;
+    const int mx = G.part.most[0], my = G.part.most[1], mz = G.part.most[2];
     const int wy = 2 * my * mz, wz = wy + 2 * mx * mz;
 #pragma unroll
     for (int j = 0; j < FACES; ++j) {
@@ -570,9 +579,9 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
         return axis == 0 ? b * sz + a * sy + l : axis == 1 ? b * sz + l * sy + a : l * sz + b * sy + a;
       };
       const int len = axis == 0 ? r.bx : axis == 1 ? r.by : r.bz;
-      const bool up = axis == 0 ? r.ix + 1 < G.px : axis == 1 ? r.iy + 1 < G.py : r.iz + 1 < G.pz;
+      const bool up = axis == 0 ? r.ix + 1 < G.part.px : axis == 1 ? r.iy + 1 < G.part.py : r.iz + 1 < G.part.pz;
       const bool down = axis == 0 ? r.ix > 0 : axis == 1 ? r.iy > 0 : r.iz > 0;
-      step[j] = (axis == 0 ? 1 : axis == 1 ? G.px : G.px * G.py) * G.face_cap;
+      step[j] = (axis == 0 ? 1 : axis == 1 ? G.part.px : G.part.px * G.part.py) * G.face_cap;
       if (up) hi[j] = uint32_t(3 * cell(len) + comp);
       if (down) lo[j] = uint32_t(3 * (cell(-1) + e0) + comp);
     }
