@@ -465,6 +465,7 @@ struct ResidentClass {
   DevBuf<int4> count;
   DevBuf<uint16_t> stride, row_ids;
   DevBuf<unsigned long long> face;   // E faces, then H faces
+  DevBuf<float2> far;                // pairs that do not fit in shared memory
   DevBuf<uint2> mon_list;
   DevBuf<int> mon_count;
   void reset() {
@@ -474,6 +475,7 @@ struct ResidentClass {
     stride.free();
     row_ids.free();
     face.free();
+    far.free();
     mon_list.free();
     mon_count.free();
   }
@@ -499,6 +501,7 @@ struct HalfClass {
 // cells below which a batch's members step together, and the most cells of such a part
 constexpr int64_t kBatchSmallRun = 40'000, kBatchSmallGradient = 256'000, kBatchCells = 1'200'000;
 
+constexpr int kResFarRows = 128;  // table rows kept in shared memory before the last pairs
 constexpr uint32_t kResSmemMax = 232448 - 4096;  // dynamic shared bytes beside the kernel's static arrays
 
 struct Engine {
@@ -694,17 +697,18 @@ struct Engine {
   // Partitions worth timing, (bricks along x, y, z, weight): per number of blocks
   // the one whose costliest brick costs least, with even cuts and with thinner
   // bricks in the layers. A brick's cost: its cells, 0.7 more per layer cell,
-  // 0.75 per face cell; its memory from the layers the split plan found. None when no
-  // partition fits. Thinner bricks take grids that even cuts do not (125x46x86
+  // 0.75 per face cell; its memory from the layers the split plan found. Where
+  // no partition fits, some pairs may stay in global memory. None when the fields
+  // alone do not fit. Thinner bricks take grids that even cuts do not (125x46x86
   // cells with 8-cell layers: half steps 14.0, here 10.7 us per step; 133x44x88
   // 15.5 -> 11.4) and even out the time (55x140x47 8.6 -> 8.0 us).
-  std::vector<std::array<int, 4>> resident_partitions(int n_sm) const {
+  std::vector<std::array<int, 4>> resident_partitions(int n_sm, bool* far_used) const {
     std::vector<std::array<int, 4>> out;
     const fdtd_sim* s = sims[0];
     const int n[3] = {s->nx, s->ny, s->nz};
     const int* t = s->split_plan.t;
     struct Part { int len, layer; };  // cells of a brick along an axis, of these in a layer
-    auto cost_of = [&](const ResPart& P) -> double {
+    auto cost_of = [&](const ResPart& P, bool far) -> double {
       std::vector<Part> kinds[3];
       const int parts[3] = {P.px, P.py, P.pz};
       for (int a = 0; a < 3; ++a)
@@ -722,17 +726,28 @@ struct Engine {
             const int v = x.len * y.len * z.len;
             auto either = [](const Part& p, const Part& q) { return p.len * q.len - (p.len - p.layer) * (q.len - q.layer); };
             const int pairs = 2 * (x.len * either(y, z) + y.len * either(x, z) + z.len * either(x, y));
-            if (res_smem(x.len, y.len, z.len, pairs) > kResSmemMax) return 1e300;
+            double over = 0;  // pairs outside shared memory
+            if (far) {
+              const uint32_t fields = res_smem(x.len, y.len, z.len, 0) + kResFarRows * kResRowBytes;
+              if (fields > kResSmemMax) return 1e300;
+              over = std::max(0.0, pairs - double(kResSmemMax - fields) / 8);
+            } else if (res_smem(x.len, y.len, z.len, pairs) > kResSmemMax) {
+              return 1e300;
+            }
             const int core = (x.len - x.layer) * (y.len - y.layer) * (z.len - z.layer);
-            worst = std::max(worst, v + 0.7 * (v - core) + 0.75 * (x.len * y.len + x.len * z.len + y.len * z.len));
+            worst = std::max(worst, v + 0.7 * (v - core) + 0.25 * over + 0.75 * (x.len * y.len + x.len * z.len + y.len * z.len));
           }
       return worst;
     };
     const bool layers = t[0] + t[1] + t[2] + t[3] + t[4] + t[5] > 0;
     ResPart P;
-    for (const int most : {n_sm, n_sm / 2, 32, 8})
+    if (24 * int64_t(n[0]) * n[1] * n[2] > int64_t(n_sm) * kResSmemMax) return out;
+    const int sizes[] = {n_sm, n_sm / 2, 32, 8, n_sm};
+    for (int k = 0; k < 5; ++k)
       for (const int thin : {0, 1}) {
-        if (thin && (!layers || most != n_sm)) continue;
+        const int most = sizes[k];
+        const bool far = k == 4;  // only where no other fits
+        if ((far && ((!out.empty() && !*far_used) || !layers)) || (thin && (!layers || most != n_sm))) continue;
         double best = 1e300;
         std::array<int, 4> pick{0, 0, 0, 0};
         for (int px = 1; px <= std::min(most, s->nx); ++px)
@@ -742,14 +757,17 @@ struct Engine {
               if (4 * px * py * pz < 3 * most && most <= s->nx * s->ny * s->nz / 64) continue;
               for (const int w : {100, 125, 150}) {
                 if ((w == 100) == (thin == 1) || !resident_cuts(s, px, py, pz, w, P)) continue;
-                const double cost = cost_of(P);
+                const double cost = cost_of(P, far);
                 if (cost < best) {
                   best = cost;
                   pick = {px, py, pz, w};
                 }
               }
             }
-        if (pick[0] && std::find(out.begin(), out.end(), pick) == out.end()) out.push_back(pick);
+        if (pick[0] && std::find(out.begin(), out.end(), pick) == out.end()) {
+          out.push_back(pick);
+          *far_used = far;
+        }
       }
     return out;
   }
@@ -786,7 +804,20 @@ struct Engine {
       state = std::max(state, res_smem(r.bx, r.by, r.bz, cnt[size_t(b)].z));
       local = std::max(local, cnt[size_t(b)].w);
     }
-    if (state > kResSmemMax) throw ArgError{FDTD_ERR_LIMIT, "Bricks do not fit in shared memory."};
+    // the pairs that do not fit beside the fields and the first rows stay in global memory
+    c.g.far = nullptr;
+    c.g.far_cap = 0;
+    if (state > kResSmemMax) {
+      state = kResSmemMax - uint32_t(std::min(local, kResFarRows)) * kResRowBytes;
+      for (int b = 0; b < nb; ++b) {
+        const ResBox r = res_box(P, b);
+        if (res_smem(r.bx, r.by, r.bz, 0) > state) throw ArgError{FDTD_ERR_LIMIT, "Bricks do not fit in shared memory."};
+        c.g.far_cap = std::max(c.g.far_cap, cnt[size_t(b)].z - res_pair_cap(r, state));
+      }
+      c.far.alloc(size_t(nb) * c.g.far_cap);
+      c.g.far = c.far.p;
+    }
+    c.g.state = state;
     const int row_cap = std::min<int>(local, int((kResSmemMax - state) / kResRowBytes));
     c.smem = state + uint32_t(row_cap) * kResRowBytes;
     const size_t nl = size_t(nb) * cells;
@@ -860,13 +891,14 @@ struct Engine {
 
   template <bool MON>
   const void* resident_variant() const {
+    if (res.g.far) return reinterpret_cast<const void*>(&res_step_kernel<4, 1024, MON, true>);
     const bool small = res.threads <= 640;  // (more registers per thread)
-    return res.faces <= 1   ? small ? reinterpret_cast<const void*>(&res_step_kernel<1, 640, MON>)
-                                    : reinterpret_cast<const void*>(&res_step_kernel<1, 1024, MON>)
-           : res.faces <= 2 ? small ? reinterpret_cast<const void*>(&res_step_kernel<2, 640, MON>)
-                                    : reinterpret_cast<const void*>(&res_step_kernel<2, 1024, MON>)
-           : small          ? reinterpret_cast<const void*>(&res_step_kernel<4, 640, MON>)
-                            : reinterpret_cast<const void*>(&res_step_kernel<4, 1024, MON>);
+    return res.faces <= 1   ? small ? reinterpret_cast<const void*>(&res_step_kernel<1, 640, MON, false>)
+                                    : reinterpret_cast<const void*>(&res_step_kernel<1, 1024, MON, false>)
+           : res.faces <= 2 ? small ? reinterpret_cast<const void*>(&res_step_kernel<2, 640, MON, false>)
+                                    : reinterpret_cast<const void*>(&res_step_kernel<2, 1024, MON, false>)
+           : small          ? reinterpret_cast<const void*>(&res_step_kernel<4, 640, MON, false>)
+                            : reinterpret_cast<const void*>(&res_step_kernel<4, 1024, MON, false>);
   }
   const void* resident_fn() const { return res.g.n_mon > 0 ? resident_variant<true>() : resident_variant<false>(); }
 
@@ -1024,8 +1056,7 @@ struct Engine {
     tune_ms = 0;
     tune_trials = 0;
     if (resident_allowed()) {
-      std::vector<TuneChoice> cand;
-      if (tune(n_sm, cand, 2)) return;
+      if (tune(n_sm, {}, 2)) return;
     }
     std::vector<TuneChoice> cand;
     for (const auto& c : kTuneCandidates) cand.push_back({c[0], c[1], c[2], c[3], c[4]});
@@ -1073,7 +1104,12 @@ struct Engine {
     if (cached && best[0] < 0) return false;  // nothing fitted
     if (cached && build(best)) return true;  // (a model of the same size may hold more split cells)
     if (variant == 2)
-      for (const auto& p : resident_partitions(n_sm)) cand.push_back({2, p[0], p[1], p[2], p[3]});
+    {
+      bool far = false;
+      for (const auto& p : resident_partitions(n_sm, &far)) cand.push_back({2, p[0], p[1], p[2], p[3]});
+      // where pairs stay in global memory the other kernels may be faster
+      if (far && !cand.empty()) cand.insert(cand.end(), {{3, 128, 0, 0, 0}, {1, 8, 6, 0, 0}, {1, 12, 4, 0, 0}});
+    }
     // (a launch of the resident kernel also loads and stores the state)
     const int warm = 2, timed = std::min(variant == 2 ? 64 : 8, nt_min - warm);
     bool found = false;
@@ -1123,6 +1159,7 @@ struct Engine {
     }
     check_error();
     tune_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (variant == 2 && best[0] != 2) found = false;  // the others' shapes are timed next
     if (!found) best[0] = -1;
     {
       std::lock_guard<std::mutex> lock(g_tune_mutex);

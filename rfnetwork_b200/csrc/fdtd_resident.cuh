@@ -11,7 +11,8 @@
 //             absorbing layers where that pays), one block each, all
 //             resident at once (cooperative launch). E and H of the brick's
 //             cells and one halo layer (H above, E below) and the split pairs
-//             of its split cells live in shared memory
+//             of its split cells live in shared memory; where these do not all
+//             fit the last of them stay in global memory (FAR)
 //   cells     two lists per brick, one in the order of the E phase and one in
 //             that of the H phase (built on the device once per simulation):
 //             first the cells whose results a neighbour waits for, then the
@@ -39,8 +40,9 @@
 // or two launches per step): 24x20x16 cells, 4-cell layers 9.0 -> 2.9 us;
 // 64x64x48, 10-cell layers 17.2 -> 5.6 us; 91x71x53 graded, 7-cell layers 20.6
 // -> 7.7 us; 100x80x64, 5-cell layers 25.8 -> 9.5 us; 133x44x88, 8-cell layers
-// (about the most that fits with such layers) 11.4 us, half steps 15.5; 120x110x80
-// without layers 22.3 -> 16.0 us. What bounds it now is a
+// 11.4 us, half steps 15.5; 120x110x80 without layers 22.3 -> 16.0 us. With some
+// pairs in global memory, against half steps: 139x49x93, 8-cell layers 17.2 -> 12.9
+// us, 120x100x64 18.7 -> 14.5; 110x100x90, 6-cell layers 22.2 us is about the most. What bounds it now is a
 // warp's chain of about a hundred dependent instructions per cell and phase
 // (about 700 cycles, two or three cells per thread), shared-memory wavefronts,
 // and two exchanges per step of about 0.6 us each, partly hidden. Two cells per
@@ -129,6 +131,9 @@ struct ResGrid {
   int n_mon, mon_cap;
   const uint2* mon_list;   // [brick][mon_cap]: field word | monitor << 16 | H side << 31, element
   const int* mon_count;    // per brick
+  uint32_t state;          // shared bytes for a brick's fields and pairs
+  float2* far;             // [brick][far_cap]: the pairs that do not fit there
+  int far_cap;
   int acc_f, acc_cap;      // phasor sums in shared memory: frequencies, elements per brick (the first of its list)
   int* err;
   uint32_t wait_limit;
@@ -451,9 +456,17 @@ __device__ __forceinline__ unsigned long long res_get(const unsigned long long* 
   return w;
 }
 
+// Pairs of a brick that fit in `state` bytes beside its fields.
+__host__ __device__ __forceinline__ int res_pair_cap(const ResBox& r, uint32_t state) {
+  return int((state - res_smem(r.bx, r.by, r.bz, 0)) / 8u);
+}
+
 // Advances steps n0 .. n1-1 of the grid. FACES: face values of one side per
 // thread (at least a brick's face values / threads). MON: with plane monitors.
-template <int FACES, int THREADS, bool MON>
+// FAR: the last pairs of a brick lie in global memory (each belongs to one thread
+// per phase, so nothing is shared through it); the addresses of all pairs are then
+// generic ones.
+template <int FACES, int THREADS, bool MON, bool FAR>
 __global__ void __launch_bounds__(THREADS, 1)
 res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
   // E quads, H quads of the local rows, then fields, pairs, phasor sums
@@ -482,7 +495,10 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
   const float4* const rows = S.rows;
   // the monitor elements whose sums stay here: nm_in of the brick's nm, sum of
   // frequency f of element i at acc[f * acc_cap + i]
-  float2* const acc = P + cnt.z;
+  const int near = FAR ? min(cnt.z, res_pair_cap(r, G.state)) : cnt.z;
+  float2* const far = FAR ? G.far + size_t(blockIdx.x) * G.far_cap : nullptr;
+  auto pair = [&](int q) -> float2& { return FAR && q >= near ? far[q - near] : P[q]; };
+  float2* const acc = P + near;
   const uint2* const ml = G.mon_list + size_t(blockIdx.x) * G.mon_cap;
   const int nm = MON ? G.mon_count[blockIdx.x] : 0, nm_in = MON ? min(nm, G.acc_cap) : 0;
   if (MON)
@@ -541,11 +557,11 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
     if (f & 63u) {
       int cs;
       const float2* const g = store_of(x, y, z, i, cs);
-      float2* p = P + (d.y & 0xffffu);
+      int p = int(d.y & 0xffffu);
       const int st = s_stride[f & 63u];
       for (int m = 0; m < 6; ++m)
         if (f >> m & 1u) {
-          *p = g[m * cs];
+          pair(p) = g[m * cs];
           p += st;
         }
     }
@@ -661,9 +677,9 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
         const int st = s_stride[f & 63u];
         const int q0 = int(d.y & 0xffffu), q1 = q0 + ((f & 1u) ? st : 0), q2 = q1 + ((f & 2u) ? st : 0);
         float2 p[3];
-        p[0] = (f & 1u) ? P[q0] : make_float2(0.f, 0.f);
-        p[1] = (f & 2u) ? P[q1] : make_float2(0.f, 0.f);
-        p[2] = (f & 4u) ? P[q2] : make_float2(0.f, 0.f);
+        p[0] = (f & 1u) ? pair(q0) : make_float2(0.f, 0.f);
+        p[1] = (f & 2u) ? pair(q1) : make_float2(0.f, 0.f);
+        p[2] = (f & 4u) ? pair(q2) : make_float2(0.f, 0.f);
         p[0].x = upd_e_split(ra.x, p[0].x, ra.y, dhz_y);  // ex_y
         p[0].y = upd_e_split(ra.z, p[0].y, ra.w, dhy_z);  // ex_z
         p[1].x = upd_e_split(rb.x, p[1].x, rb.y, dhx_z);  // ey_z
@@ -671,9 +687,9 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
         p[2].x = upd_e_split(rd.x, p[2].x, rd.y, dhy_x);  // ez_x
         p[2].y = upd_e_split(rd.z, p[2].y, rd.w, dhx_y);  // ez_y
         if (f & kResProbe) res_inject(S, __ldg(rows + 8 * (d.x >> 16) + 7), n, true, p);
-        if (f & 1u) { vx = __fadd_rn(p[0].x, p[0].y); P[q0] = p[0]; }
-        if (f & 2u) { vy = __fadd_rn(p[1].x, p[1].y); P[q1] = p[1]; }
-        if (f & 4u) { vz = __fadd_rn(p[2].x, p[2].y); P[q2] = p[2]; }
+        if (f & 1u) { vx = __fadd_rn(p[0].x, p[0].y); pair(q0) = p[0]; }
+        if (f & 2u) { vy = __fadd_rn(p[1].x, p[1].y); pair(q1) = p[1]; }
+        if (f & 4u) { vz = __fadd_rn(p[2].x, p[2].y); pair(q2) = p[2]; }
       }
       if (c < cnt.x) send(e_face, __ldg(ew + c), vx, vy, vz, uint32_t(n) + 1u);
       e[0] = vx;
@@ -731,9 +747,9 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
         const int q0 = int(d.y & 0xffffu) + __popc(f & 7u) * st, q1 = q0 + ((f & 8u) ? st : 0),
                   q2 = q1 + ((f & 16u) ? st : 0);
         float2 p[3];
-        p[0] = (f & 8u) ? P[q0] : make_float2(0.f, 0.f);
-        p[1] = (f & 16u) ? P[q1] : make_float2(0.f, 0.f);
-        p[2] = (f & 32u) ? P[q2] : make_float2(0.f, 0.f);
+        p[0] = (f & 8u) ? pair(q0) : make_float2(0.f, 0.f);
+        p[1] = (f & 16u) ? pair(q1) : make_float2(0.f, 0.f);
+        p[2] = (f & 32u) ? pair(q2) : make_float2(0.f, 0.f);
         p[0].x = upd_h_split(kx.x, p[0].x, gxy);
         p[0].y = upd_h_split(kx.z, p[0].y, gxz);
         p[1].x = upd_h_split(ky.x, p[1].x, gyz);
@@ -741,9 +757,9 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
         p[2].x = upd_h_split(kz.x, p[2].x, gzx);
         p[2].y = upd_h_split(kz.z, p[2].y, gzy);
         if (f & kResProbe) res_inject(S, __ldg(rows + 8 * (d.x >> 16) + 7), n, false, p);
-        if (f & 8u) { vx = __fadd_rn(p[0].x, p[0].y); P[q0] = p[0]; }
-        if (f & 16u) { vy = __fadd_rn(p[1].x, p[1].y); P[q1] = p[1]; }
-        if (f & 32u) { vz = __fadd_rn(p[2].x, p[2].y); P[q2] = p[2]; }
+        if (f & 8u) { vx = __fadd_rn(p[0].x, p[0].y); pair(q0) = p[0]; }
+        if (f & 16u) { vy = __fadd_rn(p[1].x, p[1].y); pair(q1) = p[1]; }
+        if (f & 32u) { vz = __fadd_rn(p[2].x, p[2].y); pair(q2) = p[2]; }
       }
       if (c < cnt.y) send(h_face, __ldg(hw + c), vx, vy, vz, uint32_t(n) + 1u);
       h[0] = vx;
@@ -799,11 +815,11 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
     if (f & 63u) {
       int cs;
       float2* const g = store_of(x, y, z, i, cs);
-      const float2* p = P + (d.y & 0xffffu);
+      int p = int(d.y & 0xffffu);
       const int st = s_stride[f & 63u];
       for (int m = 0; m < 6; ++m)
         if (f >> m & 1u) {
-          g[m * cs] = *p;
+          g[m * cs] = pair(p);
           p += st;
         }
     }
