@@ -249,6 +249,7 @@ struct fdtd_sim {
   int base_rows = 0;
   int box_rows_from = -1;
   int box_rows_box[6] = {0, 0, 0, 0, 0, 0};
+  bool uploaded = false;  // host arrays were copied since the last wait for uploads
   int generation = 0;  // bumped whenever device buffers are reallocated
 };
 
@@ -283,6 +284,7 @@ std::vector<float> record_adjoints(const fdtd_sim* s, const double* dJdX, int nt
 void h2d(fdtd_sim* s, void* dst, const void* src, size_t bytes) {
   CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
   s->h2d_bytes += int64_t(bytes);
+  s->uploaded = true;
 }
 
 void d2h(fdtd_sim* s, void* dst, const void* src, size_t bytes) {
@@ -305,14 +307,14 @@ using StreamKernelFn = void (*)(const SimDev, const SimDev*, const StreamTile*, 
 struct StreamVariant {
   int ty, threads, min_blocks, plain_blocks;
   uint32_t xch_bytes, main_bytes, split_bytes;
-  StreamKernelFn fn_of[2], plain_of[2], plain_most;  // several simulations, one
+  StreamKernelFn fn, plain_of[2], plain_most;  // plain_of: several simulations, one
 };
 
 template <int TY>
 StreamVariant stream_variant() {
   using G = StreamGeom<TY>;
   return StreamVariant{TY, G::THREADS, G::MIN_BLOCKS, G::PLAIN_BLOCKS, uint32_t(2 * G::XCH), G::MAIN, G::REGION,
-                       {&fdtd_step_stream_kernel<TY, kTilesAny, false>, &fdtd_step_stream_kernel<TY, kTilesAny, true>},
+                       &fdtd_step_stream_kernel<TY, kTilesAny, false>,
                        {&fdtd_step_stream_kernel<TY, kTilesPlain, false>, &fdtd_step_stream_kernel<TY, kTilesPlain, true>},
                        &fdtd_step_stream_kernel<TY, kTilesPlainMost, true>};
 }
@@ -537,6 +539,7 @@ struct Engine {
   int withhold = -1;                       // test hook: plane the TMA kernels' producers never issue
   bool use_graph = true;  // replay the time loop as a captured CUDA graph
   int direct_nt = -1;     // steps of the last run whose launches came from the host
+  bool uploaded = true;   // tables were copied since the last wait for uploads
   double last_ms = 0;
   double tune_ms = 0;      // host time of the autotuner's trial runs in the last tiling (0: cached choice)
   int tune_trials = 0;     // candidate shapes it timed
@@ -595,8 +598,19 @@ struct Engine {
     graph_nt = direct_nt = -1;
   }
 
+  // Waits for what this engine and its simulations uploaded, if anything.
+  void wait_uploads() {
+    bool any = uploaded;
+    for (auto* s : sims) any = any || s->uploaded;
+    if (!any) return;
+    uploads_done();
+    uploaded = false;
+    for (auto* s : sims) s->uploaded = false;
+  }
+
   void build_tiles() {
     reset_graph();
+    uploaded = true;
     cfg = asked;
     int dev = 0, n_sm = 148;
     CK(cudaGetDevice(&dev));
@@ -1178,7 +1192,7 @@ struct Engine {
     {
       c.v = find_stream_variant(cfg.ty, cfg.stages);
       if (!c.v) throw ArgError{FDTD_ERR_ARG, "No streaming kernel instantiated for this tile height / stage count."};
-      c.fn = c.v->fn_of[sims.size() == 1];
+      c.fn = c.v->fn;
       fn = reinterpret_cast<const void*>(c.fn);
       threads = c.v->threads;
       bool splits = false;
@@ -1465,6 +1479,7 @@ struct Engine {
   int n_caps = 0, cap_blocks = 1;
 
   void build_caps() {
+    uploaded = true;
     std::vector<CapSim> v;
     int64_t nb_max = 0;
     for (auto* s : sims)
@@ -2048,7 +2063,7 @@ struct Engine {
     if (!use_graph || (graph_nt != nt && direct_nt != nt)) {
       reset_graph();
       build_caps();
-      uploads_done();
+      wait_uploads();
       if (use_graph) direct_nt = nt;
       CK(cudaEventRecord(ev0, st));
       enqueue(st, nt);
@@ -2079,7 +2094,7 @@ struct Engine {
       cudaStreamDestroy(cap);
       graph_nt = nt;
     }
-    uploads_done();
+    wait_uploads();
     CK(cudaEventRecord(ev0, st));
     CK(cudaGraphLaunch(graph, st));
     CK(cudaEventRecord(ev1, st));

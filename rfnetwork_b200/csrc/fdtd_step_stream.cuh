@@ -163,7 +163,9 @@ __device__ __forceinline__ void stream_inject(const SimDev& Sd, const float4& r7
 // (fewer live registers, no split regions), and runs beside it; kTilesPlainMost
 // is the same with registers for more blocks per SM, for grids of almost only
 // plain tiles. ONE: a single simulation, whose descriptor is a kernel parameter
-// (a load from global memory per use in the plane loop otherwise).
+// (a load from global memory per use in the plane loop otherwise); for plain
+// tiles only: 256x256x128 cells with 8-cell layers take 167.6 us per step with
+// neither, 166.6 with the plain kernel so, 168.9 with both.
 enum { kTilesAny, kTilesPlain, kTilesPlainMost };
 
 template <int TY, int TILES, bool ONE>
