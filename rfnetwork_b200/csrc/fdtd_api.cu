@@ -251,6 +251,7 @@ struct fdtd_sim {
   int box_rows_box[6] = {0, 0, 0, 0, 0, 0};
   bool uploaded = false;  // host arrays were copied since the last wait for uploads
   int generation = 0;  // bumped whenever device buffers are reallocated
+  int engine_gen = -1;  // generation the simulation's own engine was built on
 };
 
 int64_t box_cells(const int* b) { return int64_t(b[1] - b[0]) * (b[3] - b[2]) * (b[5] - b[4]); }
@@ -2226,7 +2227,6 @@ void prepare(fdtd_sim* s, int nt) {
   const int nx = s->nx, ny = s->ny, nz = s->nz;
   if (!s->prepared) {
     compile_host(s);
-    ++s->generation;
     s->pitch = ((nx + 31) / 32) * 32;
     s->cells_padded = size_t(nz) * ny * s->pitch;
     if (s->cells_padded >= (size_t(1) << 31) - size_t(2) * ny * s->pitch)
@@ -2263,6 +2263,7 @@ void prepare(fdtd_sim* s, int nt) {
     s->prepared = true;
   }
   // per-nt buffers: source amplitudes, records, DFT, monitors
+  ++s->generation;
   const size_t P = s->probes.size();
   s->src.alloc(std::max<size_t>(1, P * size_t(nt)));
   s->rec.alloc(std::max<size_t>(1, P * size_t(nt)));
@@ -2408,7 +2409,12 @@ void new_engine(fdtd_sim* s) {
   s->engine->wait_limit = s->dbg_wait_limit;
   s->engine->withhold = s->dbg_withhold;
   s->engine->build_tiles();
+  s->engine_gen = s->generation;
 }
+
+// Whether s's own engine was built on the device buffers as they are: a batch
+// run of s with another number of steps moves them too.
+bool engine_current(const fdtd_sim* s) { return s->engine && s->engine_gen == s->generation; }
 
 // A gradient box must be non-empty, inside the grid and free of cells with
 // split E storage (PML slabs, source cells): the gradient treats the box
@@ -2891,9 +2897,8 @@ int fdtd_run_async(fdtd_sim* s, int nt) {
       leave_adjoint_mode(s);
       s->engine.reset();
     }
-    const bool rebuild = !s->prepared || s->prepared_nt != nt || !s->engine;
     prepare(s, nt);
-    if (rebuild) new_engine(s);
+    if (!engine_current(s)) new_engine(s);
     s->engine->run_async(nt);
     fill_stats(s, s->engine.get());
   });
@@ -2905,9 +2910,8 @@ int fdtd_run_checkpointed(fdtd_sim* s, int nt, int every) {
     if (nt < 1 || every < 1) throw ArgError{FDTD_ERR_ARG, "nt and the checkpoint interval must be positive."};
     // a re-prepared simulation has new device buffers: the engine (descriptors,
     // tensor maps, graph) must be rebuilt with it
-    const bool rebuild = !s->prepared || s->prepared_nt != nt || !s->engine || s->adj_mode != 1 ||
-                         s->ckpt_every != every || s->ckpt_nt != nt;
     prepare(s, nt);
+    const bool rebuild = !engine_current(s) || s->adj_mode != 1 || s->ckpt_every != every || s->ckpt_nt != nt;
     const size_t N = s->cells_padded;
     const size_t stride = 6 * N + (s->splits.n ? 2 * s->split_buf_pairs : 0);
     const size_t nseg = size_t((nt + every - 1) / every);
@@ -2930,10 +2934,10 @@ int fdtd_run_recorded(fdtd_sim* s, int nt, const int* box) {
   if (!s) return FDTD_ERR_ARG;
   const int rc = guarded(&s->err, [&] {
     if (nt < 1 || !box) throw ArgError{FDTD_ERR_ARG, "nt must be positive and the box given."};
-    const bool rebuild = !s->prepared || s->prepared_nt != nt || !s->engine || s->adj_mode != 2 ||
-                         s->ckpt_nt != nt || !std::equal(box, box + 6, s->adj_box);
     prepare(s, nt);
     check_gradient_box(s, box);
+    const bool rebuild = !engine_current(s) || s->adj_mode != 2 || s->ckpt_nt != nt ||
+                         !std::equal(box, box + 6, s->adj_box);
     if (rebuild) {
       leave_adjoint_mode(s);
       s->hist.alloc(size_t(nt) * 9 * size_t(box_cells(box)));

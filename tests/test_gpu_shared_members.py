@@ -1,0 +1,78 @@
+"""A simulation that runs by itself and as a member of batches: a run of one kind
+moves or frees device buffers that the engines of the other kind were built on,
+and each of them has to notice."""
+import numpy as np
+import pytest
+
+from modelgen import configs
+from rfnetwork_b200 import _lib
+from test_gpu_resident import _model_sim
+
+pytestmark = pytest.mark.gpu
+
+NT = 60
+SIZES = ((40, 36, 34), (20, 18, 16))
+PHASE = np.exp(-0.1j * np.arange(2 * NT + 1)[:, None] * np.arange(1, 3)[None]).astype(np.complex64)
+
+
+def _make(n):
+    sim, _ = _model_sim(configs.microstrip(n=n, n_pml=3, nt=2 * NT))
+    sim.add_monitor(2, 2, n[2] // 2, 1, phase=PHASE)
+    return sim
+
+
+def _results(sim):
+    return sim.probe_values(), sim.dft(), sim.monitor(0)
+
+
+def _want(n, nt):
+    sim = _make(n)
+    sim.run(nt)
+    out = _results(sim)
+    sim.close()
+    assert np.abs(out[0]).max() > 0 and np.abs(out[2]).max() > 0
+    return out
+
+
+def _same(a, b):
+    return all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("kernel", [(1, 0, 4), (1, 8, 4), (0, 0, 4)])
+def test_other_step_counts_in_between(engine_lib, kernel):
+    """Runs with another number of steps reallocate the sources, records, sums and
+    monitor outputs; the buffers between them keep the old addresses from coming back."""
+    want = {(n, nt): _want(n, nt) for n in SIZES for nt in (NT, 2 * NT)}
+    sims = [_make(n) for n in SIZES]
+    others = []
+    batch = _lib.Batch(sims)
+    batch.set_kernel(*kernel)
+    for sim in sims:
+        sim.set_kernel(*kernel)
+
+    def check(nt):
+        for n, sim in zip(SIZES, sims):
+            assert _same(_results(sim), want[n, nt])
+        other = _make(SIZES[1])  # (takes freed blocks of the records' size)
+        other.run(nt)
+        others.append(other)
+
+    for nt in (NT, NT):  # (the second run replays a graph)
+        batch.run(nt)
+        check(nt)
+    for nt in (2 * NT, NT, NT):  # by themselves
+        for sim in sims:
+            sim.run(nt)
+        check(nt)
+    batch.run(NT)  # as before, on moved buffers
+    check(NT)
+    batch.run(2 * NT)
+    check(2 * NT)
+    batch.run(NT)
+    check(NT)
+    for sim in sims:  # the same for the members' own engines
+        sim.run(NT)
+    check(NT)
+    batch.close()
+    for sim in sims + others:
+        sim.close()
