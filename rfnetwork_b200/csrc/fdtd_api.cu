@@ -2227,6 +2227,8 @@ void prepare(fdtd_sim* s, int nt) {
   const int nx = s->nx, ny = s->ny, nz = s->nz;
   if (!s->prepared) {
     compile_host(s);
+    ++s->generation;
+    s->prepared_nt = -1;
     s->pitch = ((nx + 31) / 32) * 32;
     s->cells_padded = size_t(nz) * ny * s->pitch;
     if (s->cells_padded >= (size_t(1) << 31) - size_t(2) * ny * s->pitch)
@@ -2262,8 +2264,12 @@ void prepare(fdtd_sim* s, int nt) {
     h2d(s, s->is_src.p, srcflag.data(), srcflag.size() * sizeof(int));
     s->prepared = true;
   }
+  for (const auto& m : s->monitors)
+    if (m.n_freq && m.n_phase_rows < nt / m.n_step + 1)
+      throw ArgError{FDTD_ERR_ARG, "Monitor phase table has fewer rows than nt/n_step + 1."};
   // per-nt buffers: source amplitudes, records, DFT, monitors
   ++s->generation;
+  s->prepared_nt = -1;  // until all of them are in place
   const size_t P = s->probes.size();
   s->src.alloc(std::max<size_t>(1, P * size_t(nt)));
   s->rec.alloc(std::max<size_t>(1, P * size_t(nt)));
@@ -2291,8 +2297,6 @@ void prepare(fdtd_sim* s, int nt) {
   s->mon_out.clear();
   s->mon_phase.clear();
   for (auto& m : s->monitors) {
-    if (m.n_freq && m.n_phase_rows < nt / m.n_step + 1)
-      throw ArgError{FDTD_ERR_ARG, "Monitor phase table has fewer rows than nt/n_step + 1."};
     auto out = std::make_unique<DevBuf<char>>();
     out->alloc(m.out_bytes(nt));
     auto ph = std::make_unique<DevBuf<float2>>();

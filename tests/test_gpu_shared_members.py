@@ -76,3 +76,26 @@ def test_other_step_counts_in_between(engine_lib, kernel):
     batch.close()
     for sim in sims + others:
         sim.close()
+
+
+def test_refused_step_count_in_between(engine_lib):
+    """A run refused for its step count leaves the results of the run before it, and
+    the same run again gives them again."""
+    n = SIZES[1]
+    want = _want(n, NT)
+    sim, _ = _model_sim(configs.microstrip(n=n, n_pml=3, nt=2 * NT))
+    sim.add_monitor(2, 2, n[2] // 2, 1, phase=PHASE[:NT + 1])  # too short for 2 NT steps
+    for _ in range(2):
+        sim.run(NT)
+        assert _same(_results(sim), want)
+        with pytest.raises(ValueError, match="phase table"):
+            sim.run(2 * NT)
+        sim.nt = NT
+        assert _same(_results(sim), want)
+    co = configs.microstrip(n=n, n_pml=3, nt=2 * NT).pack_inputs(gpu=True)[0]
+    sim.set_coefficients(co)  # (the refused run then compiles and moves the fields first)
+    with pytest.raises(ValueError, match="phase table"):
+        sim.run(2 * NT)
+    sim.run(NT)
+    assert _same(_results(sim), want)
+    sim.close()
