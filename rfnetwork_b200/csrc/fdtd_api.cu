@@ -2391,8 +2391,11 @@ int coef_index(const char* name) {
 
 }  // namespace
 
-// Drops what the last run kept for a gradient (snapshots or box history).
+// Drops what the last run kept for a gradient (snapshots or box history); the
+// engines whose graphs write there, or whose kernel suited the old mode, are
+// rebuilt.
 void leave_adjoint_mode(fdtd_sim* s) {
+  ++s->generation;
   s->adj_mode = 0;
   s->adj_in_batch = false;
   s->ckpt_every = 0;
@@ -2897,10 +2900,7 @@ int fdtd_run_async(fdtd_sim* s, int nt) {
   if (!s) return FDTD_ERR_ARG;
   return guarded(&s->err, [&] {
     if (nt < 1) throw ArgError{FDTD_ERR_ARG, "nt must be positive."};
-    if (s->adj_mode) {  // the time loop is captured without snapshots or history again
-      leave_adjoint_mode(s);
-      s->engine.reset();
-    }
+    if (s->adj_mode) leave_adjoint_mode(s);  // the time loop is captured without snapshots or history again
     prepare(s, nt);
     if (!engine_current(s)) new_engine(s);
     s->engine->run_async(nt);
@@ -2915,7 +2915,8 @@ int fdtd_run_checkpointed(fdtd_sim* s, int nt, int every) {
     // a re-prepared simulation has new device buffers: the engine (descriptors,
     // tensor maps, graph) must be rebuilt with it
     prepare(s, nt);
-    const bool rebuild = !engine_current(s) || s->adj_mode != 1 || s->ckpt_every != every || s->ckpt_nt != nt;
+    const bool rebuild = !engine_current(s) || s->adj_mode != 1 || s->adj_in_batch || s->ckpt_every != every ||
+                         s->ckpt_nt != nt;
     const size_t N = s->cells_padded;
     const size_t stride = 6 * N + (s->splits.n ? 2 * s->split_buf_pairs : 0);
     const size_t nseg = size_t((nt + every - 1) / every);
@@ -2940,7 +2941,7 @@ int fdtd_run_recorded(fdtd_sim* s, int nt, const int* box) {
     if (nt < 1 || !box) throw ArgError{FDTD_ERR_ARG, "nt must be positive and the box given."};
     prepare(s, nt);
     check_gradient_box(s, box);
-    const bool rebuild = !engine_current(s) || s->adj_mode != 2 || s->ckpt_nt != nt ||
+    const bool rebuild = !engine_current(s) || s->adj_mode != 2 || s->adj_in_batch || s->ckpt_nt != nt ||
                          !std::equal(box, box + 6, s->adj_box);
     if (rebuild) {
       leave_adjoint_mode(s);

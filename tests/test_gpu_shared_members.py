@@ -99,3 +99,60 @@ def test_refused_step_count_in_between(engine_lib):
     sim.run(NT)
     assert _same(_results(sim), want)
     sim.close()
+
+
+def test_modes_change_hands(engine_lib):
+    """Plain, recorded and checkpointed runs of the members by themselves and in two
+    batches, each twice (the second replays a graph) before another kind follows."""
+    boxes = [(n[0] // 2 - 4, n[0] // 2 + 4, n[1] // 2 - 3, n[1] // 2 + 3, 5, 7) for n in SIZES]
+    want, grads, others = {}, [], []
+    for n, box in zip(SIZES, boxes):
+        want[n] = _want(n, NT)
+        sim = _make(n)
+        sim.run_recorded(NT, box)
+        grads.append(sim.adjoint(2 * sim.dft(), box))
+        assert np.abs(grads[-1]).max() > 0
+        sim.close()
+    sims = [_make(n) for n in SIZES]
+    pair = [_lib.Batch(sims), _lib.Batch(sims)]
+
+    def single(mode):
+        for n, sim, box, g in zip(SIZES, sims, boxes, grads):
+            if mode == "run":
+                sim.run(NT)
+            elif mode == "recorded":
+                sim.run_recorded(NT, box)
+            else:
+                sim.run_checkpointed(NT, 16)
+            assert _same(_results(sim), want[n])
+            if mode != "run":
+                assert np.array_equal(sim.adjoint(2 * sim.dft(), box), g)
+
+    def together(batch, mode):
+        if mode == "run":
+            batch.run(NT)
+        elif mode == "recorded":
+            batch.run_recorded(NT, boxes)
+        else:
+            batch.run_checkpointed(NT, 16, boxes)
+        assert all(_same(_results(sim), want[n]) for n, sim in zip(SIZES, sims))
+        if mode != "run":
+            assert all(map(np.array_equal, batch.adjoint([2 * sim.dft() for sim in sims]), grads))
+
+    modes = ("run", "recorded", "checkpointed")
+    for a in modes:
+        for b in modes:
+            for who in (0, 1):  # who comes between: a batch, or the members by themselves
+                first = single if who == 0 else lambda m: together(pair[0], m)
+                then = (lambda m: together(pair[0], m)) if who == 0 else single
+                first(a), first(a)
+                then(b), then(b)
+                other = _make(SIZES[0])  # takes what they freed
+                other.run_recorded(NT, boxes[0])
+                others.append(other)
+                first(a), first(a)
+            together(pair[0], a), together(pair[0], a)
+            together(pair[1], b), together(pair[1], b)
+            together(pair[0], a), together(pair[1], a)
+    for x in pair + sims + others:
+        x.close()
