@@ -486,6 +486,7 @@ struct ResidentClass {
 
 // Launch shape of the half-step kernels.
 struct HalfClass {
+  int want = 0;             // threads per block asked for, within the kernels' bounds
   int threads = 0, seg = 0, rows = 0;
   dim3 grid;
   DevBuf<SimDev> d_sims;    // several simulations
@@ -974,7 +975,7 @@ struct Engine {
 
   void build_half() {
     HalfClass& c = half;
-    const int want = std::min(std::max(cfg.ty, 64), kHalfThreads) / 32 * 32;
+    const int want = c.want = std::min(std::max(cfg.ty, 64), kHalfThreads) / 32 * 32;
     if (sims.size() == 1) {
       const fdtd_sim* s = sims[0];
       half_shape(s->nx, s->ny, want, &c.seg, &c.rows);
@@ -1038,7 +1039,7 @@ struct Engine {
     }
     if (reach >= 0 && int64_t(w[2]) * int64_t(sims.size()) <= 65535) {
       L.boxes = c.d_boxes.p;
-      half_shape(w[0], w[1], std::max(64, cfg.ty), &L.seg, &L.rows);
+      half_shape(w[0], w[1], c.want, &L.seg, &L.rows);
       L.planes = w[2];
       threads = (L.seg * L.rows + 31) / 32 * 32;
       grid = dim3(unsigned((w[0] + L.seg - 1) / L.seg), unsigned((w[1] + L.rows - 1) / L.rows),

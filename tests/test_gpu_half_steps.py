@@ -112,6 +112,14 @@ def test_gradients_equal_plain(engine_lib, monkeypatch, mode):
     assert all(np.array_equal(x, y) for x, y in zip(a, b))
 
 
+# more threads per block than the kernels take, and a size that is no multiple of a
+# warp: replayed regions wide enough to use them all
+@pytest.mark.parametrize("threads", ["512", "100"])
+def test_replays_of_any_block_size(engine_lib, monkeypatch, threads):
+    monkeypatch.setenv("RFN_FDTD_TY", threads)
+    test_gradients_equal_plain(engine_lib, monkeypatch, "checkpointed")
+
+
 def test_batched_gradients_equal_single(engine_lib, monkeypatch):
     models = [configs.microstrip(n=(40, 30, 24), n_pml=4, nt=90), configs.microstrip(n=(46, 34, 22), n_pml=4, nt=90)]
     boxes = [(16, 22, 12, 17, 9, 11), (18, 24, 14, 20, 9, 12)]
