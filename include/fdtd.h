@@ -165,14 +165,17 @@ int fdtd_set_stream(fdtd_sim* s, void* stream);
  * reference's solver_run_cu does (rfnetwork/core/src/solver.cu:1005-1120). */
 int fdtd_set_graph(fdtd_sim* s, int enabled);
 
-/* Failure-path testing of the TMA streaming step kernel (variant 1), not for
- * production runs. wait_limit: sleeping polls (each at most ~2 us) after
- * which a shared-memory pipeline wait gives up (0 restores the default of
- * 2^20, about 2 s); withhold_plane >= 0: every block's producer skips the
- * loads of its plane number withhold_plane, so the waits for that plane
- * expire and the run returns FDTD_ERR_DEVICE; -1 issues every plane. The
- * next run captures its time loop again with these values. No counterpart
- * in the reference, whose kernels have no bounded waits. */
+/* Failure-path testing of the TMA streaming step kernel (variant 1) and of the
+ * resident one (variant 2), not for production runs. wait_limit: sleeping polls
+ * (each at most ~2 us; the resident kernel's eight polls count as one) after which a
+ * shared-memory pipeline wait, or the resident kernel's wait for a neighbouring
+ * brick's face value, gives up (0 restores the default of 2^20, about 2 s);
+ * withhold_plane >= 0: every block's producer skips the loads of its plane
+ * number withhold_plane, or the resident kernel's first brick sends no E faces
+ * in time step withhold_plane, so the waits for these expire and the run returns
+ * FDTD_ERR_DEVICE; -1 issues everything. The next run captures its time loop
+ * again with these values. No counterpart in the reference, whose kernels have no
+ * bounded waits. */
 int fdtd_set_debug(fdtd_sim* s, unsigned wait_limit, int withhold_plane);
 
 /* Results of the last run. out: n_probes x nt floats, probe-major. */

@@ -254,9 +254,10 @@ class Simulation:
         self._check(self.lib.fdtd_set_graph(self.h, int(bool(enabled))))
 
     def set_debug(self, wait_limit: int = 0, withhold_plane: int = -1):
-        """Failure-path testing of the streaming kernel: pipeline waits give up
+        """Failure-path testing: the streaming and resident kernels' waits give up
         after ``wait_limit`` polls (0: the default, about 2 s) and, with
-        ``withhold_plane`` >= 0, that plane's loads are never issued."""
+        ``withhold_plane`` >= 0, that plane's loads are never issued (resident
+        kernel: its first brick sends no faces in that time step)."""
         self._check(self.lib.fdtd_set_debug(self.h, int(wait_limit), int(withhold_plane)))
 
     def run(self, nt: int):

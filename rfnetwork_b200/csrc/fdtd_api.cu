@@ -21,6 +21,7 @@
 #include <string>
 #include <thread>
 #include <unordered_set>
+#include <utility>
 #include <vector>
 
 #include "../../include/fdtd.h"
@@ -465,7 +466,7 @@ struct ResidentClass {
   int threads = 0, faces = 0, blocks = 0;
   uint32_t smem = 0;
   DevBuf<uint2> lists;               // E lists, H lists, E face words, H face words
-  DevBuf<int4> count;
+  DevBuf<int4> count;                // per brick, and again for a test's launch that withholds faces
   DevBuf<uint16_t> stride, row_ids;
   DevBuf<unsigned long long> face;   // E faces, then H faces
   DevBuf<float2> far;                // pairs that do not fit in shared memory
@@ -538,7 +539,9 @@ struct Engine {
   int64_t step_launches = 0, dft_launches = 0, adj_launches = 0;
   double adj_ms = 0;
   uint32_t wait_limit = kStreamWaitLimit;  // polls per mbarrier wait of the streaming kernel
-  int withhold = -1;                       // test hook: plane the TMA kernels' producers never issue
+  // test hook: plane the TMA kernels' producers never issue, or step in which the
+  // resident kernel's first brick sends no E faces
+  int withhold = -1;
   bool use_graph = true;  // replay the time loop as a captured CUDA graph
   int direct_nt = -1;     // steps of the last run whose launches came from the host
   bool uploaded = true;   // tables were copied since the last wait for uploads
@@ -802,7 +805,7 @@ struct Engine {
     if (ResBox{0, 0, 0, bx, by, bz, 0, 0, 0}.size() * int64_t(3) >= kResNone || res_smem(bx, by, bz, 0) > kResSmemMax)
       throw ArgError{FDTD_ERR_LIMIT, "Bricks do not fit in shared memory."};
     const int n_rows = int(s->grid.rows.size());
-    c.count.alloc(size_t(nb));
+    c.count.alloc(2 * size_t(nb));
     DevBuf<int> map, nums, n_nums;
     map.alloc(size_t(nb) * n_rows);
     nums.alloc(size_t(nb) * kResScratch * cells);
@@ -813,6 +816,9 @@ struct Engine {
     CK(cudaGetLastError());
     std::vector<int4> cnt(static_cast<size_t>(nb));
     CK(cudaMemcpy(cnt.data(), c.count.p, cnt.size() * sizeof(int4), cudaMemcpyDeviceToHost));
+    const int e_faces = std::exchange(cnt[0].x, 0);
+    CK(cudaMemcpy(c.count.p + nb, cnt.data(), cnt.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    cnt[0].x = e_faces;
     int local = 0;
     uint32_t state = 0;
     for (int b = 0; b < nb; ++b) {
@@ -849,7 +855,6 @@ struct Engine {
     g.h_list = c.lists.p + nl;
     g.e_words = c.lists.p + 2 * nl;
     g.h_words = c.lists.p + 3 * nl;
-    g.count = c.count.p;
     g.row_ids = c.row_ids.p;
     g.stride = c.stride.p;
     g.e_face = c.face.p;
@@ -923,10 +928,24 @@ struct Engine {
   void launch_resident(cudaStream_t st, int n0, int n1) {
     if (n0 == 0) CK(cudaMemsetAsync(res.face.p, 0, res.face.n * sizeof(unsigned long long), st));
     res.g.s = sims[0]->dev;
-    res.g.wait_limit = wait_limit;
-    void* args[] = {&res.g, &n0, &n1};
-    CK(cudaLaunchCooperativeKernel(resident_fn(), dim3(unsigned(res.blocks)), dim3(unsigned(res.threads)), args,
-                                   res.smem, st));
+    // (its polls do not sleep and take a quarter of a microsecond: eight for one of
+    // the TMA waits', so that a limit bounds both to about the same time)
+    res.g.wait_limit = uint32_t(std::min<uint64_t>(uint64_t(wait_limit) * 8, UINT32_MAX));
+    auto launch = [&](int a, int b, const int4* count) {
+      if (a >= b) return;
+      res.g.count = count;
+      void* args[] = {&res.g, &a, &b};
+      CK(cudaLaunchCooperativeKernel(resident_fn(), dim3(unsigned(res.blocks)), dim3(unsigned(res.threads)), args,
+                                     res.smem, st));
+    };
+    const int4* const c = res.count.p;
+    if (withhold < n0 || withhold >= n1) {
+      launch(n0, n1, c);
+      return;
+    }
+    launch(n0, withhold, c);
+    launch(withhold, withhold + 1, c + res.blocks);  // (the counts with which brick 0 sends no E faces)
+    launch(withhold + 1, n1, c);
   }
 
   // Threads per row piece and rows per block of half-step blocks of at most t
@@ -2163,6 +2182,8 @@ struct Engine {
       CK(cudaMemset(d_err.p, 0, sizeof(int)));
       if (e == kErrNonFinite)
         throw ArgError{FDTD_ERR_NONFINITE, "the run diverged: a probe record or a field value is not finite"};
+      if (e == kErrFaceExpired)
+        throw ArgError{FDTD_ERR_DEVICE, "resident step kernel gave up waiting for a neighbouring brick's faces"};
       throw ArgError{FDTD_ERR_DEVICE, "step kernel gave up waiting for a TMA plane load (code " +
                                           std::to_string(e) + ")"};
     }

@@ -382,6 +382,7 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
 
 // Error codes the kernels record in the engine's error word.
 constexpr int kErrWaitExpired = 1;  // a bounded pipeline wait gave up
+constexpr int kErrFaceExpired = 3;  // a brick of the resident kernel gave up waiting for its neighbour
 constexpr int kErrNonFinite = 2;    // a probe record or a final field value is NaN or infinite
 
 // Run sentinel: records kErrNonFinite when any of n floats is NaN or

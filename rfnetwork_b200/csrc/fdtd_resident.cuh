@@ -136,7 +136,7 @@ struct ResGrid {
   int far_cap;
   int acc_f, acc_cap;      // phasor sums in shared memory: frequencies, elements per brick (the first of its list)
   int* err;
-  uint32_t wait_limit;
+  uint32_t wait_limit;     // polls per face word
 };
 
 struct ResBox {
@@ -645,7 +645,7 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
         if (hi[j] != kResNone) bad |= !receive(h_face + tid + j * T + step[j], uint32_t(n), H[hi[j]]);
     }
     if (__syncthreads_or(bad)) {
-      if (tid == 0) atomicExch(G.err, kErrWaitExpired);
+      if (tid == 0) atomicExch(G.err, kErrFaceExpired);
       return;
     }
 #pragma unroll 1
@@ -703,7 +703,7 @@ res_step_kernel(const __grid_constant__ ResGrid G, int n0, int n1) {
     for (int j = 0; j < FACES; ++j)
       if (lo[j] != kResNone) bad |= !receive(e_face + tid + j * T - step[j], uint32_t(n) + 1u, E[lo[j]]);
     if (__syncthreads_or(bad)) {
-      if (tid == 0) atomicExch(G.err, kErrWaitExpired);
+      if (tid == 0) atomicExch(G.err, kErrFaceExpired);
       return;
     }
 #pragma unroll 1

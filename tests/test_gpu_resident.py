@@ -100,6 +100,26 @@ def test_two_threads(engine_lib):
         assert len(got[k]) == 6 and all(np.array_equal(g, want[k]) for g in got[k])
 
 
+@pytest.mark.parametrize("step", [0, 7, 39])
+def test_expired_wait_reports_device_error_and_the_handle_recovers(engine_lib, step):
+    """One brick sends no faces in one step: the waits for them run out after a few
+    hundred polls, every block ends, and the same handle runs normally again."""
+    sim, nt = _model_sim(configs.microstrip(n=(40, 30, 24), n_pml=4, nt=40))
+    sim.run(nt)
+    ref, X = sim.probe_values(), sim.dft()
+    assert sim.stats()["variant"] == 2 and sim.stats()["grid"] > 1 and np.abs(ref).max() > 0
+    for _ in range(2):
+        sim.set_debug(wait_limit=200, withhold_plane=step)
+        with pytest.raises(_lib.FdtdError, match="resident step kernel gave up waiting") as e:
+            sim.run(nt)
+        assert e.value.code == 5  # FDTD_ERR_DEVICE
+        sim.set_debug()
+        for _ in range(2):
+            sim.run(nt)
+            assert np.array_equal(sim.probe_values(), ref) and np.array_equal(sim.dft(), X)
+    sim.close()
+
+
 def test_partition_follows_the_run(engine_lib):
     """A batch of one member is stepped by the resident kernel in a plain run
     and by the streaming kernels when the run records a gradient's history."""
