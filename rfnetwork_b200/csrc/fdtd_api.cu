@@ -506,6 +506,11 @@ struct HalfClass {
 // cells below which a batch's members step together, and the most cells of such a part
 constexpr int64_t kBatchSmallRun = 40'000, kBatchSmallGradient = 256'000, kBatchCells = 1'200'000;
 
+// grids whose steps fork are launched from the host below so many cells, or when a
+// monitor samples more often than every so many steps
+constexpr int64_t kDirectCells = 2'000'000;
+constexpr int kDirectSamples = 16;
+
 constexpr int kResFarRows = 128;  // table rows kept in shared memory before the last pairs
 constexpr uint32_t kResSmemMax = 232448 - 4096;  // dynamic shared bytes beside the kernel's static arrays
 
@@ -2112,15 +2117,39 @@ struct Engine {
     }
   }
 
+  // Whether a first run is faster launched from the host. The two tile lists of a
+  // streaming step, released together by the step before, start in either order
+  // when they come from the host, and where the plain tiles come first the general
+  // ones run on alone afterwards; in a graph the general ones go first. Per step
+  // and call (a graph's making included), host against graph: 256x256x128 cells with
+  // 8-cell layers 197 against 175 us, without 125 against 111; 200x180x128 without
+  // 82 against 68; 165x140x100 with 81 against 77, without 39 to 54 against 43; but
+  // 150x130x90 without 31 against 35, with 61 against 66; 130x120x80 without 27 to 38
+  // against 33. A third branch makes the graph dear (about 70 us for a step with a box
+  // history or sampled monitors beside it): 256x256x128 with monitors at every step
+  // 235 against 284 us, at every fifth 193 against 219, with a box history 182 against
+  // 250.
+  bool direct_first() const {
+    if (cfg.variant != 1 || scls.n_tiles == 0 || scls.n_tiles_p == 0) return true;
+    int64_t cells = 0;
+    for (auto* s : sims) {
+      cells += int64_t(s->nx) * s->ny * s->nz;
+      if (s->adj_mode == 2) return true;
+      for (const auto& m : s->monitors)
+        if (m.n_step < kDirectSamples) return true;
+    }
+    return cells < kDirectCells;
+  }
+
   void run_async(int nt) {
     init();
     cudaStream_t st = stream();
-    // A time loop's first run is launched from the host, its repetitions replay a
-    // graph. Making a graph, launching it the first time and destroying it costs
-    // about 5.5 us of host time per node and the GPU waits for it; a launch costs
-    // 2 us beside the steps before it (1500 half steps of 120x100x64 cells: 14 ms
-    // before the first step and 3 ms at the end, then 27 ms of steps).
-    if (!use_graph || (graph_nt != nt && direct_nt != nt)) {
+    // A time loop's first run is mostly launched from the host, its repetitions
+    // replay a graph. Making a graph, launching it the first time and destroying it
+    // costs about 5.5 us of host time per node and the GPU waits for it; a launch
+    // costs 2 us beside the steps before it (1500 half steps of 120x100x64 cells: 14
+    // ms before the first step and 3 ms at the end, then 27 ms of steps).
+    if (!use_graph || (graph_nt != nt && direct_nt != nt && direct_first())) {
       reset_graph();
       build_caps();
       wait_uploads();
