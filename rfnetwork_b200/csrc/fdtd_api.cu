@@ -510,6 +510,7 @@ constexpr int64_t kBatchSmallRun = 40'000, kBatchSmallGradient = 256'000, kBatch
 // monitor samples more often than every so many steps
 constexpr int64_t kDirectCells = 2'000'000;
 constexpr int kDirectSamples = 16;
+constexpr int kDirectLaunches = 1000;  // of a run that the caller does not wait for
 
 constexpr int kResFarRows = 128;  // table rows kept in shared memory before the last pairs
 constexpr uint32_t kResSmemMax = 232448 - 4096;  // dynamic shared bytes beside the kernel's static arrays
@@ -2129,7 +2130,11 @@ struct Engine {
   // history or sampled monitors beside it): 256x256x128 with monitors at every step
   // 235 against 284 us, at every fifth 193 against 219, with a box history 182 against
   // 250.
-  bool direct_first() const {
+  // A caller that does not wait for the run gets a graph where the launches would
+  // not fit the launch queue (1024): the call would return when most of the run is
+  // over (1500 half steps of 128x128x96 cells: after 38 of 57 ms).
+  bool direct_first(int nt, bool waits) const {
+    if (!waits && cfg.variant != 2 && int64_t(nt) * (sims[0]->monitors.empty() ? 2 : 3) > kDirectLaunches) return false;
     if (cfg.variant != 1 || scls.n_tiles == 0 || scls.n_tiles_p == 0) return true;
     int64_t cells = 0;
     for (auto* s : sims) {
@@ -2141,7 +2146,8 @@ struct Engine {
     return cells < kDirectCells;
   }
 
-  void run_async(int nt) {
+  // Enqueues a run of nt steps. waits: the caller waits for it at once.
+  void run_async(int nt, bool waits) {
     init();
     cudaStream_t st = stream();
     // A time loop's first run is mostly launched from the host, its repetitions
@@ -2149,7 +2155,7 @@ struct Engine {
     // costs about 5.5 us of host time per node and the GPU waits for it; a launch
     // costs 2 us beside the steps before it (1500 half steps of 120x100x64 cells: 14
     // ms before the first step and 3 ms at the end, then 27 ms of steps).
-    if (!use_graph || (graph_nt != nt && direct_nt != nt && direct_first())) {
+    if (!use_graph || (graph_nt != nt && direct_nt != nt && direct_first(nt, waits))) {
       reset_graph();
       build_caps();
       wait_uploads();
@@ -2573,7 +2579,7 @@ void build_batch(fdtd_batch* b, int nt) {
 void run_batch(fdtd_batch* b, int nt) {
   std::exception_ptr first;
   set_batch_streams(b);
-  for (auto& e : b->parts) e->run_async(nt);
+  for (auto& e : b->parts) e->run_async(nt, true);
   for (auto& e : b->parts) {
     try {
       e->sync();
@@ -2947,17 +2953,19 @@ int fdtd_set_stream(fdtd_sim* s, void* stream) {
   return FDTD_OK;
 }
 
-int fdtd_run_async(fdtd_sim* s, int nt) {
+static int start_run(fdtd_sim* s, int nt, bool waits) {
   if (!s) return FDTD_ERR_ARG;
   return guarded(&s->err, [&] {
     if (nt < 1) throw ArgError{FDTD_ERR_ARG, "nt must be positive."};
     if (s->adj_mode) leave_adjoint_mode(s);  // the time loop is captured without snapshots or history again
     prepare(s, nt);
     if (!engine_current(s)) new_engine(s);
-    s->engine->run_async(nt);
+    s->engine->run_async(nt, waits);
     fill_stats(s, s->engine.get());
   });
 }
+
+int fdtd_run_async(fdtd_sim* s, int nt) { return start_run(s, nt, false); }
 
 int fdtd_run_checkpointed(fdtd_sim* s, int nt, int every) {
   if (!s) return FDTD_ERR_ARG;
@@ -2979,7 +2987,7 @@ int fdtd_run_checkpointed(fdtd_sim* s, int nt, int every) {
       s->ckpt.alloc(nseg * stride);
       new_engine(s);
     }
-    s->engine->run_async(nt);
+    s->engine->run_async(nt, true);
     fill_stats(s, s->engine.get());
   });
   if (rc) return rc;
@@ -3002,7 +3010,7 @@ int fdtd_run_recorded(fdtd_sim* s, int nt, const int* box) {
       std::copy(box, box + 6, s->adj_box);
       new_engine(s);
     }
-    s->engine->run_async(nt);
+    s->engine->run_async(nt, true);
     fill_stats(s, s->engine.get());
   });
   if (rc) return rc;
@@ -3038,7 +3046,7 @@ int fdtd_synchronize(fdtd_sim* s) {
 }
 
 int fdtd_run(fdtd_sim* s, int nt) {
-  int rc = fdtd_run_async(s, nt);
+  int rc = start_run(s, nt, true);
   if (rc) return rc;
   return fdtd_synchronize(s);
 }

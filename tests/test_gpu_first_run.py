@@ -1,5 +1,7 @@
 """The first run of a time loop takes its launches from the host or from a graph,
 whichever is faster: it is not much slower than the runs that repeat it."""
+import time
+
 import numpy as np
 import pytest
 
@@ -37,3 +39,27 @@ def test_steps_of_two_tile_lists(engine_lib):
         sim.close()
     assert np.abs(records[0]).max() > 0 and all(np.array_equal(r, records[0]) for r in records)
     assert sorted(first)[-2] <= 1.15 * sorted(again)[2], (first, again)
+
+
+def test_asynchronous_run_returns_early(engine_lib, monkeypatch):
+    """More launches than the launch queue holds come from a graph when the caller does
+    not wait: the call took two thirds of the run, a graph takes a quarter of it."""
+    monkeypatch.setenv("RFN_FDTD_KERNEL", "half")
+    packed = configs.microstrip(n=(128, 128, 96), n_pml=10, nt=1500).pack_inputs(gpu=True)
+    share, records = [], []
+    for wait in (True, False, False, False):
+        sim, nt = _sim(packed)
+        sim.compile()
+        t0 = time.perf_counter()
+        if wait:
+            sim.run(nt)
+        else:
+            sim.run_async(nt)
+            t1 = time.perf_counter()
+            sim.synchronize()
+            share.append((t1 - t0) / (time.perf_counter() - t0))
+        assert sim.stats()["variant"] == 3
+        records.append(sim.probe_values())
+        sim.close()
+    assert np.abs(records[0]).max() > 0 and all(np.array_equal(r, records[0]) for r in records)
+    assert sorted(share)[1] < 0.5, share
