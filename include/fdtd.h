@@ -161,8 +161,9 @@ int fdtd_set_kernel(fdtd_sim* s, int variant, int tile_y, int stages, int zchunk
 int fdtd_set_stream(fdtd_sim* s, void* stream);
 
 /* Whether runs replay the time loop as one captured CUDA graph (enabled = 1,
- * the default) or issue every launch from the host step by step (0), as the
- * reference's solver_run_cu does (rfnetwork/core/src/solver.cu:1005-1120). */
+ * the default) or issue every launch from the host (0): step by step, as the
+ * reference's solver_run_cu does (rfnetwork/core/src/solver.cu:1005-1120), or with
+ * the resident kernel one launch for many steps. */
 int fdtd_set_graph(fdtd_sim* s, int enabled);
 
 /* Failure-path testing of the TMA streaming step kernel (variant 1) and of the

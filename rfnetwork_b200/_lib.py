@@ -250,7 +250,7 @@ class Simulation:
         self._check(self.lib.fdtd_set_stream(self.h, ctypes.c_void_p(int(stream_ptr))))
 
     def set_graph(self, enabled: bool):
-        """Replay the time loop as a CUDA graph (default) or launch every step from the host."""
+        """Replay the time loop as a CUDA graph (default) or launch everything from the host."""
         self._check(self.lib.fdtd_set_graph(self.h, int(bool(enabled))))
 
     def set_debug(self, wait_limit: int = 0, withhold_plane: int = -1):
