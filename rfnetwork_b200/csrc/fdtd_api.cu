@@ -503,8 +503,11 @@ struct HalfClass {
   }
 };
 
-// cells below which a batch's members step together, and the most cells of such a part
-constexpr int64_t kBatchSmallRun = 40'000, kBatchSmallGradient = 256'000, kBatchCells = 1'200'000;
+// A batch's members below so many cells step together in a plain run when there are
+// at least so many of them; in a gradient any number; the most cells of such a part.
+struct BatchRule { size_t members; int64_t cells; };
+constexpr BatchRule kBatchTogether[] = {{6, 90'000}, {5, 70'000}, {3, 50'000}};
+constexpr int64_t kBatchSmallGradient = 256'000, kBatchCells = 1'200'000;
 
 // grids whose steps fork are launched from the host below so many cells, or when a
 // monitor samples more often than every so many steps
@@ -2513,30 +2516,39 @@ struct fdtd_batch {
 
 // Which members step together. Members are independent, so one that fills the
 // GPU alone is best stepped alone: it takes the kernel that suits it (the
-// resident one holds up to half a million cells) and its state stays in L2,
+// resident one holds up to a million cells) and its state stays in L2,
 // while all states together do not. Eight members of 0.12 to 1.1 M cells: 151 us
 // per step together, 102 one after the other. Small members share launches,
-// whose latency is then paid once. Per member and step, together against alone,
-// 22k cells 3.7 (two members), 2.0 (four), 1.2 (32) against 3.0 us, 47k cells
-// 3.3 (four) and 2.6 (16) against 3.1 us, 85k cells 4.8 against 4.2 us. For a
-// gradient, whose steps are two or four launches: four members of 75k cells 14.9
+// whose latency is then paid once, the more the cheaper. Per member and step, in
+// parts of up to 1.2 M cells, together against alone: 22k cells 3.2 (two members),
+// 2.0 (four), 1.2 (32) against 3.2 us; 47k 3.0 (three), 2.6 (eight), 2.8 (32)
+// against 3.3; 60k 3.9 (three), 3.3 (five), 3.0 (eight), 2.9 (32) against 3.6; 85k
+// 4.9 (three), 4.2 (five), 3.9 (six), 3.7 (32) against 4.0; 110k 5.0 (three), 4.8
+// (six to 32) against 4.3; 200k 8.5 against 5.1. For a gradient, whose steps are two or four launches: four members of 75k cells 14.9
 // against 21.8 ms, 192k cells 24.8 against 28.9 ms, 346k cells 39.9 against 35.3
 // ms; six of 590k cells 96 against 78 ms.
 std::vector<std::vector<size_t>> batch_parts(const fdtd_batch* b) {
   std::vector<std::vector<size_t>> out;
-  std::vector<size_t> small;
+  std::vector<size_t> small;  // members that step together
   auto cells = [&](size_t i) { return int64_t(b->sims[i]->nx) * b->sims[i]->ny * b->sims[i]->nz; };
   const bool automatic = b->asked.variant == 1 && b->asked.ty == 0, run = b->sims[0]->adj_mode == 0;
-  for (size_t i = 0; i < b->sims.size(); ++i) {
-    if (!automatic || cells(i) < (run ? kBatchSmallRun : kBatchSmallGradient))
-      small.push_back(i);
-    else
-      out.push_back({i});
+  auto below = [&](int64_t limit) {
+    std::vector<size_t> v;
+    for (size_t i = 0; i < b->sims.size(); ++i)
+      if (!automatic || cells(i) < limit) v.push_back(i);
+    return v;
+  };
+  if (!automatic || !run) {
+    small = below(kBatchSmallGradient);
+  } else {
+    for (const auto& r : kBatchTogether)
+      if (small.empty() && below(r.cells).size() >= r.members) small = below(r.cells);
   }
+  for (size_t i = 0; i < b->sims.size(); ++i)
+    if (!std::binary_search(small.begin(), small.end(), i)) out.push_back({i});
   int64_t room = 0;
   for (size_t i : small) {
-    const bool together = !automatic || !run || small.size() > 2;
-    if (!together || (automatic && room < cells(i)) || room == 0) {
+    if ((automatic && room < cells(i)) || room == 0) {
       out.emplace_back();
       room = kBatchCells;
     }

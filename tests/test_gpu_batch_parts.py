@@ -47,3 +47,32 @@ def test_members_keep_their_bits(engine_lib, members):
     batch.close()
     for sim in sims:
         sim.close()
+
+
+@pytest.mark.parametrize("members,together", [
+    ([SMALL] * 2, False), ([SMALL] * 3, True), ([MID] * 2, False), ([MID] * 3, True), ([MID] * 8, True),
+    ([(46, 40, 33)] * 4, False), ([(46, 40, 33)] * 5, True), ([(52, 44, 37)] * 5, False), ([(52, 44, 37)] * 6, True),
+    ([LARGE] * 6, False), ([MID, (52, 44, 37)] * 3 + [LARGE], True)])
+def test_the_more_the_larger(engine_lib, members, together):
+    """Members of 50k to 90k cells are stepped together only where they are many: the
+    first part's kernel is the resident one where each is stepped alone."""
+    models = {n: _model_sim(configs.microstrip(n=n, n_pml=3, nt=NT)) for n in set(members)}
+    want = {}
+    for n, (sim, _) in models.items():
+        sim.run(NT)
+        want[n] = sim.probe_values()
+        sim.close()
+    sims = [_model_sim(configs.microstrip(n=n, n_pml=3, nt=NT))[0] for n in members]
+    batch = _lib.Batch(sims)
+    batch.run(NT)
+    tiles = batch.stats()["n_tiles"]
+    alone = 0
+    for n, sim in zip(members, sims):
+        assert np.abs(want[n]).max() > 0 and np.array_equal(sim.probe_values(), want[n])
+        sim.run(NT)
+        assert sim.stats()["variant"] == 2
+        alone += sim.stats()["n_tiles"]
+    assert (tiles != alone) == together
+    batch.close()
+    for sim in sims:
+        sim.close()
