@@ -625,6 +625,7 @@ struct Engine {
   void build_tiles() {
     reset_graph();
     uploaded = true;
+    n_caps = 0;  // (a kept engine's last run may have recorded)
     cfg = asked;
     int dev = 0, n_sm = 148;
     CK(cudaGetDevice(&dev));
@@ -1089,9 +1090,10 @@ struct Engine {
   int state_buf(int n) const { return cfg.variant >= 2 ? 0 : n & 1; }
 
   // Picks the step kernel and its shape for this set of grids: each candidate
-  // runs a few time steps on the simulations themselves (their fields are
-  // cleared again by the next run), the fastest is kept and remembered for the
-  // same grid sizes. A grid whose state fits in shared memory takes the
+  // runs a few time steps on the simulations themselves, with the monitors and the
+  // box histories that these keep (all is cleared or written again by the next
+  // run), the fastest is kept and remembered for the same grid sizes and the same
+  // work beside the steps. A grid whose state fits in shared memory takes the
   // resident kernel, whose partitions are timed (from 24x20x16 to 120x110x80
   // cells it takes a third to three quarters of the streaming kernels' time per
   // step, the least gain at the largest that fits); the others the streaming
@@ -1116,6 +1118,18 @@ struct Engine {
       key.insert(key.end(), {s->nx, s->ny, s->nz});
       nt_min = std::min(nt_min, s->prepared_nt);
     }
+    // box histories, and the monitors' elements per step and cell in octaves: kernels
+    // differ in what these cost them (the resident kernel samples inside, the half
+    // steps write the histories themselves and wait for the samples)
+    double sampled = 0, cells = 0;
+    bool recorded = false;
+    for (auto* s : sims) {
+      recorded = recorded || s->adj_mode == 2;
+      cells += double(s->nx) * s->ny * s->nz;
+      for (const auto& m : s->monitors) sampled += double(m.n1) * m.n2 * std::max(1, m.n_freq) / m.n_step;
+    }
+    key.push_back(recorded);
+    key.push_back(sampled > 0 ? int(std::floor(std::log2(sampled / cells))) : INT_MIN);
     // (what fits in shared memory depends on the layers)
     if (variant == 2) key.insert(key.end(), sims[0]->split_plan.t, sims[0]->split_plan.t + 6);
     const KernelConfig auto_cfg = cfg;
@@ -1128,6 +1142,7 @@ struct Engine {
       cfg.one_list = c[4];
       try {
         build_shape(n_sm);
+        build_caps();
       } catch (const ArgError& e) {
         cfg = auto_cfg;
         if (e.code != FDTD_ERR_LIMIT) throw;
@@ -1443,15 +1458,17 @@ struct Engine {
     return int(c.n_tiles > 0) + int(c.n_tiles_p > 0);
   }
 
-  // Time steps n0 .. n1-1 on st; returns how many launches that took, a launch
-  // of the resident kernel counted once per step.
+  // Time steps n0 .. n1-1 on st as a run has them; returns how many launches that
+  // took, a launch of the resident kernel counted once per step.
   int launch_steps(cudaStream_t st, int n0, int n1) {
     if (cfg.variant == 2) {
       launch_resident(st, n0, n1);
       return n1 - n0;
     }
     int k = 0;
-    for (int n = n0; n < n1; ++n) k += launch_step(st, n);
+    bool mon_pending = false;
+    for (int n = n0; n < n1; ++n) k += step_and_samples(st, n, mon_pending);
+    if (mon_pending) CK(cudaStreamWaitEvent(st, mon_join, 0));
     return k;
   }
 
@@ -2013,6 +2030,55 @@ struct Engine {
     }
   }
 
+  // Step n with what a run takes from it: the box histories and the monitors'
+  // samples. mon_pending: the samples are not waited for yet. Returns the step
+  // kernels launched.
+  int step_and_samples(cudaStream_t st, int n, bool& mon_pending) {
+    int k = 0;
+    if (cfg.variant == 3) {  // the E launch writes the box history of its step
+      launch_half(st, n, false, n_caps > 0);
+      launch_half(st, n, true, false);
+      k = 1;
+    } else if (n_caps) {
+      // the box history of step n reads buffer n & 1, which step n only
+      // reads and step n+1 overwrites: it runs on a side stream beside step n
+      CK(cudaEventRecord(cap_fork, st));
+      CK(cudaStreamWaitEvent(cap_stream, cap_fork, 0));
+      adj_capture_kernel<<<dim3(cap_blocks, unsigned(n_caps)), 256, 0, cap_stream>>>(d_caps.p, n, 0);
+      CK(cudaGetLastError());
+      CK(cudaEventRecord(cap_join, cap_stream));
+    }
+    if (cfg.variant != 3) k = launch_step(st, n);
+    if (n_caps && cfg.variant != 3) CK(cudaStreamWaitEvent(st, cap_join, 0));
+    // The monitors of step n read the buffer that step n + 1 only reads: they
+    // run on a side stream beside it, and step n + 2, which overwrites that
+    // buffer, waits for them. (The half steps work in place: there the next
+    // step waits.)
+    if (mon_pending) {
+      CK(cudaStreamWaitEvent(st, mon_join, 0));
+      mon_pending = false;
+    }
+    bool sample = false;
+    for (auto* s : sims)
+      for (const auto& m : s->monitors) sample = sample || monitor_samples(n, m.n_step);
+    if (sample) {
+      CK(cudaEventRecord(mon_fork, st));
+      CK(cudaStreamWaitEvent(mon_stream, mon_fork, 0));
+      for (auto* s : sims)
+        if (!s->monitors.empty()) {
+          int most = 1;
+          for (const auto& m : s->monitors) most = std::max(most, m.n1 * m.n2);
+          monitor_kernel<<<dim3(unsigned(std::min(64, (most + 127) / 128)), unsigned(s->monitors.size())), 128, 0,
+                           mon_stream>>>(s->d_dev.p, s->d_mons.p, n, state_buf(n + 1));
+          CK(cudaGetLastError());
+        }
+      CK(cudaEventRecord(mon_join, mon_stream));
+      mon_pending = cfg.variant != 3;
+      if (!mon_pending) CK(cudaStreamWaitEvent(st, mon_join, 0));
+    }
+    return k;
+  }
+
   // Enqueue one full run of nt steps on stream st (used for capture and for
   // direct launches alike).
   void enqueue(cudaStream_t st, int nt) {
@@ -2064,47 +2130,7 @@ struct Engine {
           if (sb)
             CK(cudaMemcpyAsync(dst + 6 * N, s->splits.p + b * sb, sb * sizeof(float), cudaMemcpyDeviceToDevice, st));
         }
-      if (cfg.variant == 3) {  // the E launch writes the box history of its step
-        launch_half(st, n, false, n_caps > 0);
-        launch_half(st, n, true, false);
-        ++step_launches;
-      } else if (n_caps) {
-        // the box history of step n reads buffer n & 1, which step n only
-        // reads and step n+1 overwrites: it runs on a side stream beside step n
-        CK(cudaEventRecord(cap_fork, st));
-        CK(cudaStreamWaitEvent(cap_stream, cap_fork, 0));
-        adj_capture_kernel<<<dim3(cap_blocks, unsigned(n_caps)), 256, 0, cap_stream>>>(d_caps.p, n, 0);
-        CK(cudaGetLastError());
-        CK(cudaEventRecord(cap_join, cap_stream));
-      }
-      if (cfg.variant != 3) step_launches += launch_step(st, n);
-      if (n_caps && cfg.variant != 3) CK(cudaStreamWaitEvent(st, cap_join, 0));
-      // The monitors of step n read the buffer that step n + 1 only reads: they
-      // run on a side stream beside it, and step n + 2, which overwrites that
-      // buffer, waits for them. (The half steps work in place: there the next
-      // step waits.)
-      if (mon_pending) {
-        CK(cudaStreamWaitEvent(st, mon_join, 0));
-        mon_pending = false;
-      }
-      bool sample = false;
-      for (auto* s : sims)
-        for (const auto& m : s->monitors) sample = sample || monitor_samples(n, m.n_step);
-      if (sample) {
-        CK(cudaEventRecord(mon_fork, st));
-        CK(cudaStreamWaitEvent(mon_stream, mon_fork, 0));
-        for (auto* s : sims)
-          if (!s->monitors.empty()) {
-            int most = 1;
-            for (const auto& m : s->monitors) most = std::max(most, m.n1 * m.n2);
-            monitor_kernel<<<dim3(unsigned(std::min(64, (most + 127) / 128)), unsigned(s->monitors.size())), 128, 0,
-                             mon_stream>>>(s->d_dev.p, s->d_mons.p, n, state_buf(n + 1));
-            CK(cudaGetLastError());
-          }
-        CK(cudaEventRecord(mon_join, mon_stream));
-        mon_pending = cfg.variant != 3;
-        if (!mon_pending) CK(cudaStreamWaitEvent(st, mon_join, 0));
-      }
+      step_launches += step_and_samples(st, n, mon_pending);
       if ((n + 1) % kDftChunk == 0 || n + 1 == nt) dft_upto(n + 1);
     }
     if (mon_pending) CK(cudaStreamWaitEvent(st, mon_join, 0));
