@@ -159,7 +159,7 @@ struct KernelConfig {
 constexpr int kTuneCandidates[][5] = {{1, 8, 6, 0, 0}, {1, 8, 8, 0, 0},  {1, 8, 4, 0, 0}, {1, 8, 6, 32, 0},
                                       {1, 12, 4, 0, 0}, {1, 6, 6, 0, 0}, {1, 4, 6, 0, 0}, {1, 4, 6, 16, 0},
                                       {1, 8, 6, 4, 0}, {1, 4, 6, 4, 0},  {1, 8, 6, 0, 1}, {1, 8, 6, 4, 1},
-                                      {1, 4, 6, 4, 1}, {3, 128, 0, 0, 0}, {3, 256, 0, 0, 0}};
+                                      {1, 4, 6, 4, 1}, {3, 256, 0, 0, 0}, {3, 128, 0, 0, 0}};
 using TuneChoice = std::array<int, 5>;
 std::mutex g_tune_mutex;
 std::map<std::vector<int>, TuneChoice> g_tune_cache;
@@ -523,6 +523,8 @@ struct Engine {
   KernelConfig asked;      // as set by the caller (may leave the choice to the autotuner)
   KernelConfig cfg;        // the kernel in use
   StreamClass scls;        // streaming kernel
+  // split cells of each simulation's boxes, while tiles are built (the same for every shape timed)
+  std::vector<std::unique_ptr<GradedIndex>> split_index;
   ResidentClass res;       // resident kernel
   HalfClass half;          // half-step kernels
   DevBuf<SimDev> d_sims;   // plain kernel
@@ -634,12 +636,13 @@ struct Engine {
       d_err.alloc(1);
       CK(cudaMemset(d_err.p, 0, sizeof(int)));
     }
-    if (cfg.variant == 1 && cfg.ty == 0) {
-      autotune(n_sm);
-      return;
-    }
     if (cfg.variant != 0) {
-      build_shape(n_sm);
+      split_index.clear();
+      if (cfg.variant == 1 && cfg.ty == 0)
+        autotune(n_sm);
+      else
+        build_shape(n_sm);
+      split_index.clear();
       return;
     }
     // plain kernel: 31 x 7 tiles, z cut into chunks
@@ -1180,30 +1183,28 @@ struct Engine {
     const auto t0 = std::chrono::steady_clock::now();
     init();
     cudaStream_t st = stream();
-    // time per step of one candidate over `steps` steps, < 0 when it does not fit
+    // time per step of one candidate over `steps` steps, < 0 when it does not fit:
+    // the resident kernel's launches as they are, the others' steps over a replayed
+    // graph, as repeated runs launch them (from the host the two kernels of a step
+    // start in either order, up to 40 % apart)
     auto trial = [&](const TuneChoice& c, int steps) -> float {
       if (!build(c)) return -1.f;
       uploads_done();
-      if (scls.d_counter.n) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), st));
-      launch_steps(st, 0, warm);
-      CK(cudaEventRecord(ev0, st));
-      launch_steps(st, warm, warm + steps);
-      CK(cudaEventRecord(ev1, st));
-      CK(cudaStreamSynchronize(st));
       float ms = 0;
-      CK(cudaEventElapsedTime(&ms, ev0, ev1));
       ++tune_trials;
-      return ms / float(steps);
-    };
-    // the same over a replayed graph, as repeated runs launch the steps
-    auto trial_graph = [&](const TuneChoice& c, int steps) -> float {
-      if (!build(c)) return -1.f;
-      uploads_done();
+      if (cfg.variant == 2) {
+        launch_steps(st, 0, warm);
+        CK(cudaEventRecord(ev0, st));
+        launch_steps(st, warm, warm + steps);
+        CK(cudaEventRecord(ev1, st));
+        CK(cudaStreamSynchronize(st));
+        CK(cudaEventElapsedTime(&ms, ev0, ev1));
+        return ms / float(steps);
+      }
       cudaStream_t cap;
       cudaGraph_t g = nullptr;
       cudaGraphExec_t ge = nullptr;
       CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-      float ms = 0;
       try {
         CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
         if (scls.d_counter.n) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), cap));
@@ -1228,27 +1229,38 @@ struct Engine {
       cudaGraphExecDestroy(ge);
       cudaGraphDestroy(g);
       cudaStreamDestroy(cap);
-      ++tune_trials;
       return ms / float(steps);
     };
     std::vector<std::pair<float, TuneChoice>> timing;
+    float least = 0;  // of the steps timed so far
+    // a look takes about so many ms of steps once a step's time is known
+    auto steps_in = [&](float ms, int fewest, int most) {
+      return least > 0 ? std::max(fewest, std::min(most, int(ms / least))) : most;
+    };
+    // the half steps with half as many threads are at most a sixth faster
+    auto hopeless = [&](const TuneChoice& c) {
+      return c[0] == 3 && !timing.empty() && timing.back().second[0] == 3 && timing.back().first > 1.2f * least;
+    };
     for (const auto& c : cand) {
-      const float ms = trial(c, timed);
-      if (ms >= 0.f) timing.emplace_back(ms, c);
+      if (hopeless(c)) continue;
+      const float ms = trial(c, c[0] == 2 ? timed : std::min(steps_in(0.5f, 4, 8), nt_min));
+      if (ms < 0.f) continue;
+      timing.emplace_back(ms, c);
+      least = least > 0 ? std::min(least, ms) : ms;
     }
     std::stable_sort(timing.begin(), timing.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
     found = !timing.empty();
     if (found) best = timing[0].second;
-    // eight launched steps tell shapes apart to a few percent (the fork and join of
-    // two tile lists cost up to 10 % more than in a graph): the best four of those
-    // within 10 % are timed again as repeated runs are. 150x130x90 cells without
-    // layers, 400 steps, over models and processes: 10.4 to 13.5 ms with the first
-    // look's choice
-    if (variant != 2 && timing.size() > 1 && timing[1].first < 1.10f * timing[0].first) {
+    // few steps tell shapes apart to a percent or two: the best three of those within
+    // 2 % are timed again over more. (150x130x90 cells without layers, 400 steps, over
+    // models and processes: 10.4 to 13.5 ms with a first look's choice from launched
+    // steps.)
+    if (variant != 2 && timing.size() > 1 && timing[1].first < 1.02f * timing[0].first) {
+      const int steps = std::min(steps_in(1.f, 6, 24), nt_min);
       float best_ms = 1e30f;
-      for (size_t k = 0; k < std::min<size_t>(4, timing.size()); ++k) {
-        if (timing[k].first >= 1.10f * timing[0].first) break;
-        const float ms = trial_graph(timing[k].second, std::min(24, nt_min));
+      for (size_t k = 0; k < std::min<size_t>(3, timing.size()); ++k) {
+        if (timing[k].first >= 1.02f * timing[0].first) break;
+        const float ms = trial(timing[k].second, steps);
         if (ms >= 0.f && ms < best_ms) {
           best_ms = ms;
           best = timing[k].second;
@@ -1305,7 +1317,8 @@ struct Engine {
       zchunk_used = std::min(zchunk_used, zc);
       c.host_maps.emplace_back();
       encode_stream_maps(c.host_maps.back(), s, ty);
-      const GradedIndex split_idx(s->grid, kFlagESplit | kFlagHSplit);
+      if (split_index.size() <= i) split_index.push_back(std::make_unique<GradedIndex>(s->grid, kFlagESplit | kFlagHSplit));
+      const GradedIndex& split_idx = *split_index[i];
       // z chunks of at most zc planes that do not straddle a z slab's inner
       // face: the first core chunk starts one plane past the low slab (its
       // halo plane is then a core plane), so interior columns of core chunks

@@ -71,3 +71,25 @@ def test_tuning_after_a_recorded_run(engine_lib, members):
     batch.close()
     for sim in sims:
         sim.close()
+
+
+def test_tuning_takes_a_few_hundred_steps(engine_lib):
+    """A first call on a size that no tuned one shares pays for the trials: two thirds
+    of the time of 400 steps of these grids, two thirds more than that when every trial
+    made its index of the split cells anew and ran forty steps and more."""
+    cost = []
+    for n in ((200, 180, 128), (202, 178, 127), (198, 182, 129)):
+        co, pr, mo, mem, Nx, Ny, Nz, Nt = configs.boxes(n=n, n_pml=8, n_boxes=8, nt=100, n_ports=2,
+                                                        n_probes=4).pack_inputs(gpu=True)
+        sim = _lib.Simulation(Nx, Ny, Nz)
+        sim.set_coefficients(co, borrow=True)
+        for p in pr:
+            sim.add_probe(p["field"], p["idx"], p["is_source"], p["values"][:Nt] if p["is_source"] else None)
+        sim.run(Nt)
+        st = sim.stats()
+        assert st["tune_trials"] > 10
+        for _ in range(2):
+            sim.run(Nt)
+        cost.append(st["tune_ms"] / (sim.stats()["last_run_ms"] / Nt))
+        sim.close()
+    assert min(cost) < 400, cost
