@@ -64,6 +64,32 @@ __host__ __device__ __forceinline__ int64_t box_cell(int x, int y, int z, int bn
   return (int64_t(z) * bny + y) * bnx + x;
 }
 
+// Box arrays with x fastest (box_cell) into the caller's order, z fastest: n arrays
+// of bnx x bny x bnz, one 32 x 32 tile of (x, z) per block and pass through shared
+// memory. (On the host the strided reads of a box of 80 x 80 x 50 cells took 12 ms
+// beside a sweep of 4 ms; here 0.1 ms, and the copy 1.6.)
+constexpr int kBoxTile = 32;
+
+__global__ void __launch_bounds__(kBoxTile * 8)
+adj_turn_kernel(const double* __restrict__ src, double* __restrict__ dst, int bnx, int bny, int bnz, int n) {
+  __shared__ double t[kBoxTile][kBoxTile + 1];
+  const int64_t nb = int64_t(bnx) * bny * bnz;
+  const int x0 = blockIdx.x * kBoxTile, z0 = blockIdx.y * kBoxTile;
+  for (int r = blockIdx.z; r < n * bny; r += gridDim.z) {
+    const int k = r / bny, y = r - k * bny;
+    for (int j = threadIdx.y; j < kBoxTile; j += blockDim.y) {
+      const int x = x0 + threadIdx.x, z = z0 + j;
+      if (x < bnx && z < bnz) t[j][threadIdx.x] = src[k * nb + box_cell(x, y, z, bnx, bny)];
+    }
+    __syncthreads();
+    for (int j = threadIdx.y; j < kBoxTile; j += blockDim.y) {
+      const int x = x0 + j, z = z0 + threadIdx.x;
+      if (x < bnx && z < bnz) dst[k * nb + (int64_t(x) * bny + y) * bnz + z] = t[threadIdx.x][j];
+    }
+    __syncthreads();
+  }
+}
+
 // Box history of one simulation at one step: E^n and the six H differences
 // the E update of step n uses.
 struct CapSim {

@@ -2027,20 +2027,22 @@ struct Engine {
     CK(cudaEventElapsedTime(&ms, ev0, ev1));
     adj_ms = ms;
     check_error();
-    // the device's box arrays run x fastest, the caller's z fastest
-    std::vector<double> g;
+    // the device's box arrays run x fastest, the caller's z fastest; three of the nine
+    // arrays at a time are turned into the adjoint state's place (24 bytes per cell)
     for (size_t i = 0; i < req.size(); ++i) {
       const int* b = req[i].box;
       const int bx = b[1] - b[0], by = b[3] - b[2], bz = b[5] - b[4];
-      g.resize(adj_bufs[i]->grad.n);
-      CK(cudaMemcpy(g.data(), adj_bufs[i]->grad.p, g.size() * sizeof(double), cudaMemcpyDeviceToHost));
-      double* out = req[i].grad_out;
-      for (int k = 0; k < 9; ++k, out += box_cells(b))
-        for (int x = 0; x < bx; ++x)
-          for (int y = 0; y < by; ++y)
-            for (int z = 0; z < bz; ++z)
-              out[(size_t(x) * by + y) * bz + z] = g[size_t(k) * size_t(box_cells(b)) + size_t(box_cell(x, y, z, bx, by))];
+      const size_t nb = size_t(box_cells(b));
+      double* const turned = reinterpret_cast<double*>(adj_bufs[i]->lam.p);
+      for (size_t k = 0; k < 9; k += 3) {
+        const dim3 grid(unsigned((bx + kBoxTile - 1) / kBoxTile), unsigned((bz + kBoxTile - 1) / kBoxTile),
+                        unsigned(std::min(3 * by, 65535)));
+        adj_turn_kernel<<<grid, dim3(kBoxTile, 8), 0, st>>>(adj_bufs[i]->grad.p + k * nb, turned, bx, by, bz, 3);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(req[i].grad_out + k * nb, turned, 3 * nb * sizeof(double), cudaMemcpyDeviceToHost, st));
+      }
     }
+    CK(cudaStreamSynchronize(st));
   }
 
   // Step n with what a run takes from it: the box histories and the monitors'
