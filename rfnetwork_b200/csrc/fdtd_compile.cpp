@@ -71,7 +71,9 @@ using RowMap = std::unordered_map<Row, uint32_t, RowHash, RowEq>;
 
 // d[z] = 0 where the coefficients of the n cells from `at` equal those of the
 // cells from `ref` bit for bit.
+#if defined(__x86_64__)  // (other hosts, such as the Arm one of a Grace-Blackwell node, have no such targets)
 __attribute__((target_clones("avx512f", "avx2", "default")))
+#endif
 void column_differences(const float* const* coef, int64_t at, int64_t ref, int n, uint32_t* d) {
   typedef uint32_t __attribute__((may_alias)) word;
   for (int z = 0; z < n; ++z) d[z] = 0;
