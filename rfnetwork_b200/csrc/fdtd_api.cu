@@ -505,9 +505,11 @@ struct HalfClass {
 
 // A batch's members below so many cells step together in a plain run when there are
 // at least so many of them; in a gradient any number; the most cells of such a part.
+// Members of a gradient of so many cells and more share launches again.
 struct BatchRule { size_t members; int64_t cells; };
 constexpr BatchRule kBatchTogether[] = {{6, 90'000}, {5, 70'000}, {3, 50'000}};
-constexpr int64_t kBatchSmallGradient = 256'000, kBatchCells = 1'200'000;
+constexpr int64_t kBatchSmallGradient = 256'000, kBatchLargeGradient = 3'500'000,
+                  kBatchCells = 1'200'000;
 
 // grids whose steps fork are launched from the host below so many cells, or when a
 // monitor samples more often than every so many steps
@@ -2567,7 +2569,10 @@ struct fdtd_batch {
 // 4.9 (three), 4.2 (five), 3.9 (six), 3.7 (32) against 4.0; 110k 5.0 (three), 4.8
 // (six to 32) against 4.3; 200k 8.5 against 5.1. For a gradient, whose steps are two or four launches: four members of 75k cells 14.9
 // against 21.8 ms, 192k cells 24.8 against 28.9 ms, 346k cells 39.9 against 35.3
-// ms; six of 590k cells 96 against 78 ms.
+// ms; six of 590k cells 96 against 78 ms; two of 2.3 M 36 against 34 ms. From where
+// the reverse step no longer works in L2 the members' shared launches only save
+// their ends: two of 3.5 M cells 50 against 50 ms, of 4.6 M 62 against 66 (without
+// layers 48 against 55), of 8.4 M 100 against 104.
 std::vector<std::vector<size_t>> batch_parts(const fdtd_batch* b) {
   std::vector<std::vector<size_t>> out;
   std::vector<size_t> small;  // members that step together
@@ -2585,8 +2590,17 @@ std::vector<std::vector<size_t>> batch_parts(const fdtd_batch* b) {
     for (const auto& r : kBatchTogether)
       if (small.empty() && below(r.cells).size() >= r.members) small = below(r.cells);
   }
-  for (size_t i = 0; i < b->sims.size(); ++i)
-    if (!std::binary_search(small.begin(), small.end(), i)) out.push_back({i});
+  int large = -1;  // the part of a gradient's largest members
+  for (size_t i = 0; i < b->sims.size(); ++i) {
+    if (std::binary_search(small.begin(), small.end(), i)) continue;
+    const bool shares = !run && cells(i) >= kBatchLargeGradient;
+    if (shares && large >= 0) {
+      out[size_t(large)].push_back(i);
+    } else {
+      if (shares) large = int(out.size());
+      out.push_back({i});
+    }
+  }
   int64_t room = 0;
   for (size_t i : small) {
     if ((automatic && room < cells(i)) || room == 0) {

@@ -76,3 +76,44 @@ def test_the_more_the_larger(engine_lib, members, together):
     batch.close()
     for sim in sims:
         sim.close()
+
+
+def test_largest_members_of_a_gradient_share_launches(engine_lib):
+    """Two members whose reverse step does not fit in L2: their adjoints together took
+    35 ms against 41 one after the other; each keeps the bits of its own."""
+    n, nt, box = (200, 180, 128), 60, (100, 116, 150, 166, 53, 57)
+    m = configs.boxes(n=n, n_pml=0, n_boxes=8, nt=nt, n_ports=2, n_probes=4)
+    packed = m.pack_inputs(gpu=True)
+    small = _model_sim(configs.microstrip(n=SMALL, n_pml=3, nt=nt))[0]
+
+    def make():
+        sim = _lib.Simulation(*n)
+        sim.set_coefficients(packed[0], borrow=True)
+        for p in packed[1]:
+            sim.add_probe(p["field"], p["idx"], p["is_source"], p["values"][:nt] if p["is_source"] else None)
+        sim.set_dft([(k % 3, k, 1.0) for k in range(len(packed[1]))], np.linspace(0.01, 0.4, 7))
+        return sim
+
+    sims = [make(), make()]
+    alone, grads = [], []
+    for sim in sims:
+        for _ in range(3):
+            sim.run_recorded(nt, box)
+            g = sim.adjoint(2 * sim.dft(), box)
+        alone.append(sim.stats()["adjoint_ms"])
+        grads.append(g)
+    assert np.abs(grads[0]).max() > 0
+    members = [sims[0], small, sims[1]]
+    batch = _lib.Batch(members)
+    for _ in range(3):
+        batch.run_recorded(nt, [box, BOXES[SMALL], box])
+        got = batch.adjoint([2 * sim.dft() for sim in members])
+    together = batch.stats()["adjoint_ms"]
+    assert np.array_equal(got[0], grads[0]) and np.array_equal(got[2], grads[1])
+    small.run_recorded(nt, BOXES[SMALL])
+    assert np.array_equal(got[1], small.adjoint(2 * small.dft(), BOXES[SMALL]))
+    # (the small member's own part adds its 0.5 ms)
+    assert together - small.stats()["adjoint_ms"] < 0.93 * sum(alone), (together, alone)
+    batch.close()
+    for sim in members:
+        sim.close()
