@@ -2029,19 +2029,21 @@ struct Engine {
     CK(cudaEventElapsedTime(&ms, ev0, ev1));
     adj_ms = ms;
     check_error();
-    // the device's box arrays run x fastest, the caller's z fastest; three of the nine
-    // arrays at a time are turned into the adjoint state's place (24 bytes per cell)
+    // the device's box arrays run x fastest, the caller's z fastest; they are turned
+    // into the adjoint state's place (24 bytes per cell), three at a time when the box
+    // is larger than a third of the grid
     for (size_t i = 0; i < req.size(); ++i) {
       const int* b = req[i].box;
       const int bx = b[1] - b[0], by = b[3] - b[2], bz = b[5] - b[4];
       const size_t nb = size_t(box_cells(b));
       double* const turned = reinterpret_cast<double*>(adj_bufs[i]->lam.p);
-      for (size_t k = 0; k < 9; k += 3) {
+      const int per = 9 * nb * sizeof(double) <= adj_bufs[i]->lam.n * sizeof(float) ? 9 : 3;
+      for (size_t k = 0; k < 9; k += size_t(per)) {
         const dim3 grid(unsigned((bx + kBoxTile - 1) / kBoxTile), unsigned((bz + kBoxTile - 1) / kBoxTile),
-                        unsigned(std::min(3 * by, 65535)));
-        adj_turn_kernel<<<grid, dim3(kBoxTile, 8), 0, st>>>(adj_bufs[i]->grad.p + k * nb, turned, bx, by, bz, 3);
+                        unsigned(std::min(per * by, 65535)));
+        adj_turn_kernel<<<grid, dim3(kBoxTile, 8), 0, st>>>(adj_bufs[i]->grad.p + k * nb, turned, bx, by, bz, per);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(req[i].grad_out + k * nb, turned, 3 * nb * sizeof(double), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(req[i].grad_out + k * nb, turned, per * nb * sizeof(double), cudaMemcpyDeviceToHost, st));
       }
     }
     CK(cudaStreamSynchronize(st));

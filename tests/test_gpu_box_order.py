@@ -6,6 +6,7 @@ import pytest
 
 from modelgen import configs
 from rfnetwork_b200 import _lib
+from rfnetwork_b200.solver_constants import COEFF_NAMES
 
 pytestmark = pytest.mark.gpu
 
@@ -35,7 +36,8 @@ def _free(sources, want, n):
 def test_parts_of_a_box(engine_lib):
     """A cell's gradient does not depend on the box around it: boxes of one cell, of a
     tile (32) and one cell more and less along x and z are the same bits as their part
-    of a large one."""
+    of a large one. (The arrays are turned at once, or three by three when the box is
+    larger than a third of the grid.)"""
     n, nt = (96, 90, 88), 240
     sim, sources = _sim(n, nt)
     big = _free(sources, (67, 24, 66), n)
@@ -69,3 +71,26 @@ def test_large_boxes_cost_the_host_a_copy(engine_lib):
         rest.append((wall - sim.stats()["adjoint_ms"]) / sim.stats()["adjoint_ms"])
     sim.close()
     assert sorted(rest)[2] < 1.2, rest
+
+
+def test_a_box_of_most_of_the_grid(engine_lib):
+    """The box fills more than a third of the grid: the same bits as a part of it by
+    itself."""
+    n, nt = (24, 26, 30), 50
+    rng = np.random.default_rng(7)
+    sim = _lib.Simulation(*n)
+    for name in COEFF_NAMES:
+        a = np.full(n, 0.97) if name[0] + name[1] in ("Ca", "Da") else np.full(n, 0.3)
+        sim.set_coefficient(name, a.astype(np.float32))
+    sim.add_probe(2, (12, 2, 14), True, rng.standard_normal(nt).astype(np.float32))
+    sim.add_probe(2, (12, 23, 14))
+    sim.set_dft([(0, 1, 1.0)], [0.1, 0.3])
+    big = (1, 23, 4, 25, 1, 29)
+    sim.run_recorded(nt, big)
+    dJ = 2 * sim.dft()
+    want = sim.adjoint(dJ, big)
+    assert (np.abs(want) > 0).mean() > 0.5
+    box = (3, 4, 6, 20, 2, 29)
+    sim.run_recorded(nt, box)
+    assert np.array_equal(sim.adjoint(dJ, box), want[:, :, 2:3, 2:16, 1:28])
+    sim.close()
