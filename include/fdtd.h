@@ -143,14 +143,16 @@ int fdtd_synchronize(fdtd_sim* s);
  * per tile (0: derived from the grid). tile_y = 0 with variant 1 autotunes:
  * the first run times a few candidate (tile_y, stages, zchunk, one or two
  * tile lists) shapes on the simulation itself for a few steps and keeps the
- * fastest, remembered per set of grid sizes for the life of the process. A
- * single grid whose state fits in the GPU's shared memory, without monitors
- * and without anything kept for a gradient, is then stepped by the resident
- * kernel (one cooperative launch for many steps; its partitions are timed);
- * for the others the half-step kernels (E, then H, in place) are candidates
- * too, which RFN_FDTD_KERNEL=half asks for. The
- * default comes from RFN_FDTD_KERNEL (plain / stream) / RFN_FDTD_TY /
- * RFN_FDTD_STAGES / RFN_FDTD_ZCHUNK or is (1, 0, 6, 0): autotuned streaming.
+ * fastest, remembered per set of grid sizes and per work beside the steps
+ * (monitors, a gradient's box history) for the life of the process. A single
+ * grid whose fields fit in the GPU's shared memory (about a million cells) and
+ * that keeps nothing for a gradient is stepped by the resident kernel where that
+ * is the fastest (one cooperative launch for many steps, plane monitors
+ * included; its partitions are timed, and the other kernels beside it when some
+ * split pairs do not fit); for the others the half-step kernels (E, then H, in
+ * place) are candidates too. The default comes from RFN_FDTD_KERNEL (plain /
+ * stream / half) / RFN_FDTD_TY / RFN_FDTD_STAGES / RFN_FDTD_ZCHUNK or is
+ * (1, 0, 6, 0): autotuned.
  * RFN_FDTD_ONE_LIST=1 sends the plain tiles of an explicit streaming shape
  * through the general kernel (one launch per step instead of two).
  * All variants give bit-identical results. The reference has one fixed 8x8x8
@@ -228,19 +230,20 @@ int fdtd_set_box_coefficients(fdtd_sim* s, const int* box, const float* coefs);
  *   grad   3 x 3 x box cells doubles, [component ex ey ez][Ca, Cb1, Cb2][x][y][z]:
  *          dJ/d(Ca_e*), dJ/d(first Cb_e*), dJ/d(second Cb_e*) in the coefficient
  *          dict's order (Ca_ex_y with Ca_ex_z held equal, Cb_ex_y, Cb_ex_z, ...)
- * The discrete adjoint runs backwards from the last step, one kernel launch
- * per step, with the transposed update in FP32 and the products accumulated in
- * FP64. Its work buffers (about 36 floats per cell) stay allocated on the
- * simulation for the next call until fdtd_destroy. */
+ * The discrete adjoint runs backwards from the last step, one kernel launch per
+ * step or two in place where its state fits in L2, with the transposed update in
+ * FP32 and the products accumulated in FP64. Its work buffers (about 36 floats per
+ * cell, in place 18) stay allocated on the simulation for the next call until
+ * fdtd_destroy. */
 int fdtd_adjoint(fdtd_sim* s, const double* dJ_dX, int n_series, int n_freq, const int* box, double* grad);
 
 /* ---------------------------------------------------------------- batches */
 
 /* Many independent simulations of uneven sizes run by one call. Small members
- * step together, one launch covering the work lists of them all; members that
- * fill the GPU alone run one after the other (a kernel chosen with
- * fdtd_batch_set_kernel steps all members together). The time loops are captured
- * as CUDA graphs. The statistics count a step of all members as one launch.
+ * step together where they are many, one launch covering the work lists of them
+ * all; members that fill the GPU alone run one after the other, except the largest
+ * of a gradient (a kernel chosen with fdtd_batch_set_kernel steps all members
+ * together). Repeated time loops replay CUDA graphs. The statistics count a step of all members as one launch.
  * The reference has no batched engine; its
  * counterpart is one solver_run_cu call per simulation
  * (rfnetwork/core/src/cuda_binding.cpp:20-68). Members keep their own
