@@ -1235,9 +1235,10 @@ struct Engine {
     };
     std::vector<std::pair<float, TuneChoice>> timing;
     float least = 0;  // of the steps timed so far
-    // a look takes about so many ms of steps once a step's time is known
+    // a look takes about so many ms of steps once a step's time is known (many short
+    // ones, so that a graph's own start of some microseconds counts little)
     auto steps_in = [&](float ms, int fewest, int most) {
-      return least > 0 ? std::max(fewest, std::min(most, int(ms / least))) : most;
+      return least > 0 ? std::max(fewest, std::min(most, int(ms / least))) : 8;
     };
     // the half steps with half as many threads are at most a sixth faster
     auto hopeless = [&](const TuneChoice& c) {
@@ -1245,7 +1246,7 @@ struct Engine {
     };
     for (const auto& c : cand) {
       if (hopeless(c)) continue;
-      const float ms = trial(c, c[0] == 2 ? timed : std::min(steps_in(0.5f, 4, 8), nt_min));
+      const float ms = trial(c, c[0] == 2 ? timed : std::min(steps_in(0.3f, 4, 32), nt_min));
       if (ms < 0.f) continue;
       timing.emplace_back(ms, c);
       least = least > 0 ? std::min(least, ms) : ms;
@@ -1258,7 +1259,7 @@ struct Engine {
     // models and processes: 10.4 to 13.5 ms with a first look's choice from launched
     // steps.)
     if (variant != 2 && timing.size() > 1 && timing[1].first < 1.02f * timing[0].first) {
-      const int steps = std::min(steps_in(1.f, 6, 24), nt_min);
+      const int steps = std::min(steps_in(0.6f, 6, 48), nt_min);
       float best_ms = 1e30f;
       for (size_t k = 0; k < std::min<size_t>(3, timing.size()); ++k) {
         if (timing[k].first >= 1.02f * timing[0].first) break;
