@@ -2644,6 +2644,7 @@ void build_batch(fdtd_batch* b, int nt) {
     e->build_tiles();
   }
   b->run_nt = nt;
+  b->dirty = false;  // (a call refused before this leaves a chosen kernel for the next)
 }
 
 // Runs nt steps of every part and reports the first error after all have ended.
@@ -3227,7 +3228,6 @@ int fdtd_batch_run(fdtd_batch* b, int nt) {
   return guarded(&b->err, [&] {
     if (nt < 1) throw ArgError{FDTD_ERR_ARG, "nt must be positive."};
     bool rebuild = b->run_nt != nt || b->parts.empty() || b->dirty;
-    b->dirty = false;
     for (auto* s : b->sims) {
       if (!s->prepared || s->prepared_nt != nt) rebuild = true;
       if (s->adj_mode) {
@@ -3276,7 +3276,6 @@ int fdtd_batch_run_recorded(fdtd_batch* b, int nt, const int* boxes) {
   return guarded(&b->err, [&] {
     if (nt < 1 || !boxes) throw ArgError{FDTD_ERR_ARG, "nt must be positive and the boxes given."};
     bool rebuild = b->run_nt != nt || b->parts.empty() || b->dirty;
-    b->dirty = false;
     for (size_t i = 0; i < b->sims.size(); ++i) {
       fdtd_sim* s = b->sims[i];
       const int* box = boxes + 6 * i;
@@ -3314,7 +3313,6 @@ int fdtd_batch_run_checkpointed(fdtd_batch* b, int nt, int every, const int* box
     if (nt < 1 || every < 1 || !boxes)
       throw ArgError{FDTD_ERR_ARG, "nt and the checkpoint interval must be positive and the boxes given."};
     bool rebuild = b->run_nt != nt || b->parts.empty() || b->dirty;
-    b->dirty = false;
     const size_t nseg = size_t((nt + every - 1) / every);
     for (size_t i = 0; i < b->sims.size(); ++i) {
       fdtd_sim* s = b->sims[i];

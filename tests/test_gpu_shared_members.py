@@ -156,3 +156,22 @@ def test_modes_change_hands(engine_lib):
             together(pair[0], a), together(pair[1], a)
     for x in pair + sims + others:
         x.close()
+
+
+def test_kernel_chosen_before_a_refused_call(engine_lib):
+    """A batch call refused for one member's box does not forget the kernel chosen
+    before it."""
+    sims = [_make(n) for n in SIZES]
+    batch = _lib.Batch(sims)
+    batch.run(NT)
+    assert batch.stats()["variant"] != 0
+    want = [_results(sim) for sim in sims]
+    batch.set_kernel(0)
+    with pytest.raises(ValueError, match="box"):
+        batch.run_recorded(NT, [(0, 3, 0, 3, 0, 3), (4, 6, 4, 6, 5, 7)])
+    batch.run(NT)
+    assert batch.stats()["variant"] == 0
+    assert all(_same(_results(sim), w) for sim, w in zip(sims, want))
+    batch.close()
+    for sim in sims:
+        sim.close()
