@@ -74,9 +74,9 @@ def test_tuning_after_a_recorded_run(engine_lib, members):
 
 
 def test_tuning_takes_a_few_hundred_steps(engine_lib):
-    """A first call on a size that no tuned one shares pays for the trials: two thirds
-    of the time of 400 steps of these grids, two thirds more than that when every trial
-    made its index of the split cells anew and ran forty steps and more."""
+    """A first call on a size that no tuned one shares pays for the trials: the time of
+    300 to 350 steps of these grids, and of 680 to 760 when every trial made its index
+    of the split cells anew and ran more steps. The bound lies between."""
     cost = []
     for n in ((200, 180, 128), (202, 178, 127), (198, 182, 129)):
         co, pr, mo, mem, Nx, Ny, Nz, Nt = configs.boxes(n=n, n_pml=8, n_boxes=8, nt=100, n_ports=2,
@@ -92,4 +92,4 @@ def test_tuning_takes_a_few_hundred_steps(engine_lib):
             sim.run(Nt)
         cost.append(st["tune_ms"] / (sim.stats()["last_run_ms"] / Nt))
         sim.close()
-    assert min(cost) < 400, cost
+    assert min(cost) < 520, cost
