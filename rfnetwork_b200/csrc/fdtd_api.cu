@@ -300,6 +300,18 @@ void d2h(fdtd_sim* s, void* dst, const void* src, size_t bytes) {
 // comes between the uploads and the first kernel on another stream.
 void uploads_done() { CK(cudaStreamSynchronize(0)); }
 
+// Lets a kernel be launched with as much dynamic shared memory as a block can have.
+// The limit belongs to the function, not to a launch: set to what one engine uses,
+// it made the launches of another engine that uses more fail.
+void allow_shared(const void* fn) {
+  int dev = 0, most = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  cudaFuncAttributes a{};
+  CK(cudaFuncGetAttributes(&a, fn));
+  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(a.sharedSizeBytes)));
+}
+
 using StreamKernelFn = void (*)(const SimDev, const SimDev*, const StreamTile*, int, int, unsigned*, unsigned, int*, int, int,
                                 uint32_t, int);
 
@@ -917,7 +929,7 @@ struct Engine {
     c.faces = (nf + c.threads - 1) / c.threads;
     c.blocks = nb;
     const void* fn = resident_fn();
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kResSmemMax)));
+    allow_shared(fn);
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, c.threads, c.smem));
     if (per_sm < 1) throw ArgError{FDTD_ERR_LIMIT, "Resident kernel does not fit on an SM."};
@@ -1300,7 +1312,7 @@ struct Engine {
       smem = int(c.ring);
       ty = c.v->ty;
     }
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    allow_shared(fn);
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
     if (per_sm < 1) throw ArgError{FDTD_ERR_LIMIT, "Step kernel does not fit on an SM."};
@@ -1413,7 +1425,7 @@ struct Engine {
       int no_regions = 0;
       c.ring_p = stream_slots(*c.v, cfg.stages, plain_blocks, false, &c.n_main_p, &no_regions);
       const void* fp = reinterpret_cast<const void*>(c.fn_plain);
-      CK(cudaFuncSetAttribute(fp, cudaFuncAttributeMaxDynamicSharedMemorySize, int(c.ring_p)));
+      allow_shared(fp);
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_p, fp, threads, int(c.ring_p)));
       if (per_sm_p < 1) throw ArgError{FDTD_ERR_LIMIT, "Step kernel does not fit on an SM."};
       per_sm_p = std::min(per_sm_p, plain_blocks);
@@ -1813,7 +1825,7 @@ struct Engine {
       if (adj_slots < 3) throw ArgError{FDTD_ERR_LIMIT, "Streaming reverse step's plane slots do not fit."};
       adj_smem = uint32_t(adj_slots) * AG::SLOT;
       const void* fn = reinterpret_cast<const void*>(&adj_stream_kernel<kAdjStreamTileY>);
-      CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(adj_smem)));
+      allow_shared(fn);
       int per_sm = 0;
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, AG::THREADS, int(adj_smem)));
       if (per_sm < 1) throw ArgError{FDTD_ERR_LIMIT, "Streaming reverse step does not fit on an SM."};

@@ -1,6 +1,7 @@
 """A simulation that runs by itself and as a member of batches: a run of one kind
 moves or frees device buffers that the engines of the other kind were built on,
-and each of them has to notice."""
+and each of them has to notice. And several engines side by side, each with its own
+shape of the same kernels."""
 import numpy as np
 import pytest
 
@@ -174,4 +175,32 @@ def test_kernel_chosen_before_a_refused_call(engine_lib):
     assert all(_same(_results(sim), w) for sim, w in zip(sims, want))
     batch.close()
     for sim in sims:
+        sim.close()
+
+
+def test_handles_with_different_plane_slots(engine_lib):
+    """Handles whose launches use different amounts of shared memory take turns; each
+    runs from the host first and as a graph later, and a gradient's replays too."""
+    n, box = SIZES[0], (16, 24, 14, 20, 9, 11)
+    want = _want(n, NT)
+    sims = []
+    for stages in (8, 4, 6, 3):
+        sim = _make(n)
+        sim.set_kernel(1, 8, stages)
+        sims.append(sim)
+    for _ in range(3):
+        for sim in sims:
+            sim.run(NT)
+            assert _same(_results(sim), want)
+    grads = []
+    for _ in range(2):
+        for sim in sims:
+            sim.run_checkpointed(NT, 16)
+        for sim in sims:
+            grads.append(sim.adjoint(2 * sim.dft(), box))
+    assert np.abs(grads[0]).max() > 0 and all(np.array_equal(g, grads[0]) for g in grads)
+    for sim in sims:
+        sim.set_graph(False)
+        sim.run(NT)
+        assert _same(_results(sim), want)
         sim.close()
