@@ -18,6 +18,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <shared_mutex>
 #include <string>
 #include <thread>
 #include <unordered_set>
@@ -88,6 +89,69 @@ cudaMemPool_t engine_pool() {
   return pools[dev];
 }
 
+// A wait for the whole device and a capture in another thread spoil each other:
+// the wait is refused and the capture ends invalid. Captures share this lock, waits
+// take it alone.
+std::shared_mutex& capture_mutex() {
+  static std::shared_mutex m;
+  return m;
+}
+
+cudaError_t device_wait() {
+  std::unique_lock<std::shared_mutex> lock(capture_mutex());
+  const cudaError_t e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) cudaGetLastError();  // (the next launch's check is not to find it)
+  return e;
+}
+
+// An instantiated graph (null: none).
+struct Graph {
+  cudaGraphExec_t exec = nullptr;
+  Graph() = default;
+  explicit Graph(cudaGraphExec_t e) : exec(e) {}
+  Graph(Graph&& o) noexcept : exec(std::exchange(o.exec, nullptr)) {}
+  Graph& operator=(Graph&& o) noexcept {
+    std::swap(exec, o.exec);
+    return *this;
+  }
+  ~Graph() {
+    if (exec) cudaGraphExecDestroy(exec);
+  }
+};
+
+// What f launches on the stream it is given, as a graph; none when the capture was
+// ended by a wait for the device outside this library.
+template <typename F>
+Graph capture(F&& f) {
+  cudaStream_t cap;
+  cudaGraph_t g = nullptr;
+  CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+  try {
+    std::shared_lock<std::shared_mutex> lock(capture_mutex());
+    CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
+    f(cap);
+    CK(cudaStreamEndCapture(cap, &g));
+  } catch (const CudaError& e) {
+    cudaStreamEndCapture(cap, &g);
+    if (g) cudaGraphDestroy(g);
+    cudaStreamDestroy(cap);
+    cudaGetLastError();
+    if (e.code == cudaErrorStreamCaptureInvalidated) return Graph();
+    throw;
+  } catch (...) {
+    cudaStreamEndCapture(cap, &g);
+    if (g) cudaGraphDestroy(g);
+    cudaStreamDestroy(cap);
+    throw;
+  }
+  cudaStreamDestroy(cap);
+  cudaGraphExec_t exec = nullptr;
+  const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
+  cudaGraphDestroy(g);
+  CK(e);
+  return Graph(exec);
+}
+
 template <typename T>
 struct DevBuf {
   T* p = nullptr;
@@ -107,8 +171,10 @@ struct DevBuf {
     n = count;
   }
   void free() {
-    if (p) {
-      cudaDeviceSynchronize();  // no stream may still use it (cudaFree would wait the same way)
+    // no stream may still use it (cudaFree would wait the same way); where the wait is
+    // refused, because code outside this library captures a stream, the block stays out
+    // of use
+    if (p && device_wait() == cudaSuccess) {
       cudaFreeAsync(p, 0);
       cudaStreamSynchronize(0);
     }
@@ -549,7 +615,7 @@ struct Engine {
   int zchunk_used = 0;
   cudaStream_t own_stream = nullptr;
   cudaStream_t ext_stream = nullptr;
-  cudaGraphExec_t graph = nullptr;
+  Graph graph;
   int graph_nt = -1;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaStream_t cap_stream = nullptr;                   // box-history captures beside the steps
@@ -602,7 +668,6 @@ struct Engine {
     }
   }
   ~Engine() {
-    if (graph) cudaGraphExecDestroy(graph);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (cap_fork) cudaEventDestroy(cap_fork);
@@ -623,8 +688,7 @@ struct Engine {
   }
 
   void reset_graph() {
-    if (graph) cudaGraphExecDestroy(graph);
-    graph = nullptr;
+    graph = Graph();
     graph_nt = direct_nt = -1;
   }
 
@@ -1215,34 +1279,23 @@ struct Engine {
         CK(cudaEventElapsedTime(&ms, ev0, ev1));
         return ms / float(steps);
       }
-      cudaStream_t cap;
-      cudaGraph_t g = nullptr;
-      cudaGraphExec_t ge = nullptr;
-      CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-      try {
-        CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-        if (scls.d_counter.n) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), cap));
-        launch_steps(cap, 0, steps);
-        CK(cudaStreamEndCapture(cap, &g));
-        CK(cudaGraphInstantiate(&ge, g, 0));
-        CK(cudaGraphLaunch(ge, st));
-        CK(cudaEventRecord(ev0, st));
-        CK(cudaGraphLaunch(ge, st));
-        CK(cudaEventRecord(ev1, st));
-        CK(cudaStreamSynchronize(st));
-        CK(cudaEventElapsedTime(&ms, ev0, ev1));
-      } catch (...) {
-        cudaGraph_t dummy = nullptr;
-        cudaStreamEndCapture(cap, &dummy);
-        if (dummy) cudaGraphDestroy(dummy);
-        if (ge) cudaGraphExecDestroy(ge);
-        if (g) cudaGraphDestroy(g);
-        cudaStreamDestroy(cap);
-        throw;
-      }
-      cudaGraphExecDestroy(ge);
-      cudaGraphDestroy(g);
-      cudaStreamDestroy(cap);
+      auto steps_from_zero = [&](cudaStream_t on) {
+        if (scls.d_counter.n) CK(cudaMemsetAsync(scls.d_counter.p, 0, scls.d_counter.n * sizeof(unsigned), on));
+        launch_steps(on, 0, steps);
+      };
+      const Graph g = capture(steps_from_zero);
+      auto once = [&] { 
+        if (g.exec)
+          CK(cudaGraphLaunch(g.exec, st));
+        else
+          steps_from_zero(st);
+      };
+      once();
+      CK(cudaEventRecord(ev0, st));
+      once();
+      CK(cudaEventRecord(ev1, st));
+      CK(cudaStreamSynchronize(st));
+      CK(cudaEventElapsedTime(&ms, ev0, ev1));
       return ms / float(steps);
     };
     std::vector<std::pair<float, TuneChoice>> timing;
@@ -2217,43 +2270,23 @@ struct Engine {
     // costs about 5.5 us of host time per node and the GPU waits for it; a launch
     // costs 2 us beside the steps before it (1500 half steps of 120x100x64 cells: 14
     // ms before the first step and 3 ms at the end, then 27 ms of steps).
-    if (!use_graph || (graph_nt != nt && direct_nt != nt && direct_first(nt, waits))) {
+    bool direct = !use_graph || (graph_nt != nt && direct_nt != nt && direct_first(nt, waits));
+    if (direct || graph_nt != nt) {
       reset_graph();
       build_caps();
-      wait_uploads();
-      if (use_graph) direct_nt = nt;
-      CK(cudaEventRecord(ev0, st));
-      enqueue(st, nt);
-      CK(cudaEventRecord(ev1, st));
-      timing_pending = true;
-      return;
     }
-    if (graph_nt != nt) {
-      reset_graph();
-      build_caps();
-      cudaStream_t cap;
-      CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-      cudaGraph_t g = nullptr;
-      try {
-        CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-        enqueue(cap, nt);
-        CK(cudaStreamEndCapture(cap, &g));
-        CK(cudaGraphInstantiate(&graph, g, 0));
-      } catch (...) {
-        cudaGraph_t dummy = nullptr;
-        cudaStreamEndCapture(cap, &dummy);
-        if (dummy) cudaGraphDestroy(dummy);
-        if (g) cudaGraphDestroy(g);
-        cudaStreamDestroy(cap);
-        throw;
-      }
-      cudaGraphDestroy(g);
-      cudaStreamDestroy(cap);
-      graph_nt = nt;
+    if (!direct && graph_nt != nt) {
+      graph = capture([&](cudaStream_t cap) { enqueue(cap, nt); });
+      direct = !graph.exec;
+      if (!direct) graph_nt = nt;
     }
     wait_uploads();
+    if (direct && use_graph) direct_nt = nt;
     CK(cudaEventRecord(ev0, st));
-    CK(cudaGraphLaunch(graph, st));
+    if (direct)
+      enqueue(st, nt);
+    else
+      CK(cudaGraphLaunch(graph.exec, st));
     CK(cudaEventRecord(ev1, st));
     timing_pending = true;
   }
@@ -2370,7 +2403,7 @@ void prepare(fdtd_sim* s, int nt) {
       CK(cudaMemset(s->mat.p, 0, N * 2));
       transpose_ids_kernel<<<1024, 256>>>(tmp.p, s->mat.p, nx, ny, nz, s->pitch);
       CK(cudaGetLastError());
-      CK(cudaDeviceSynchronize());
+      CK(device_wait());
     }
     s->rows.alloc(s->grid.rows.size() * 8);
     h2d(s, s->rows.p, s->grid.rows.data(), s->grid.rows.size() * sizeof(Row));
@@ -2811,7 +2844,7 @@ void set_box_coefficients(fdtd_sim* s, const int* box, const float* coefs) {
     set_box_ids_kernel<<<256, 256>>>(s->mat.p, s->ny, s->pitch, box[0], box[2], box[4], box[1] - box[0], bny, bnz,
                                      tmp.p);
     CK(cudaGetLastError());
-    CK(cudaDeviceSynchronize());
+    CK(device_wait());
   }
 }
 
@@ -3410,7 +3443,7 @@ int fdtd_trim_memory(int64_t keep_bytes, int64_t* reserved, int64_t* used) {
     if (keep_bytes < 0) throw ArgError{FDTD_ERR_ARG, "fdtd_trim_memory: keep_bytes must be >= 0"};
     cudaMemPool_t pool = engine_pool();
     // blocks freed by destroyed simulations are returned once every stream is past their last use
-    CK(cudaDeviceSynchronize());
+    CK(device_wait());
     CK(cudaMemPoolTrimTo(pool, size_t(keep_bytes)));
     uint64_t r = 0, u = 0;
     CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &r));
