@@ -126,24 +126,23 @@ Graph capture(F&& f) {
   cudaStream_t cap;
   cudaGraph_t g = nullptr;
   CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+  std::shared_lock<std::shared_mutex> lock(capture_mutex());
   try {
-    std::shared_lock<std::shared_mutex> lock(capture_mutex());
     CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
     f(cap);
     CK(cudaStreamEndCapture(cap, &g));
-  } catch (const CudaError& e) {
-    cudaStreamEndCapture(cap, &g);
+  } catch (...) {
+    // (an ended capture shows as different errors in what is captured after it)
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(cap, &status);
+    const cudaError_t end = cudaStreamEndCapture(cap, &g);
     if (g) cudaGraphDestroy(g);
     cudaStreamDestroy(cap);
     cudaGetLastError();
-    if (e.code == cudaErrorStreamCaptureInvalidated) return Graph();
-    throw;
-  } catch (...) {
-    cudaStreamEndCapture(cap, &g);
-    if (g) cudaGraphDestroy(g);
-    cudaStreamDestroy(cap);
+    if (status == cudaStreamCaptureStatusInvalidated || end == cudaErrorStreamCaptureInvalidated) return Graph();
     throw;
   }
+  lock.unlock();
   cudaStreamDestroy(cap);
   cudaGraphExec_t exec = nullptr;
   const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);

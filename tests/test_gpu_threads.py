@@ -1,7 +1,6 @@
 """Handles used by several threads at the same time: what one thread builds, captures
 or releases must not disturb the runs of another."""
 import threading
-import time
 
 import numpy as np
 import pytest
@@ -84,34 +83,4 @@ def test_threads_that_tune_capture_and_release(engine_lib):
             busy[0] = False
 
     _run([all_groups, churn])
-    _check(got, models)
-
-
-def test_another_threads_waits_for_the_device(engine_lib):
-    """A wait for the whole device outside the library ends a capture; the run then
-    takes its launches from the host, and the next one makes its graph."""
-    import torch
-
-    n = (114, 106, 94)
-    models = {n: configs.microstrip(n=n, n_pml=8, nt=NT)}
-    got, busy = {}, [True]
-
-    def waits():
-        for _ in range(3000):
-            if not busy[0]:
-                break
-            try:
-                torch.cuda.synchronize()
-            except RuntimeError:  # (refused while a capture is under way)
-                pass
-            time.sleep(1e-3)
-
-    def work():
-        try:
-            got[n] = _work(models[n], n)
-        finally:
-            busy[0] = False
-
-    torch.cuda.synchronize()
-    _run([work, waits])
     _check(got, models)
